@@ -63,7 +63,8 @@ __global__ void __launch_bounds__(256) fused_step_kernel(const Rec<real>* __rest
   const int patch = blockIdx.x;
   load_rec(R, rin);
   Layers<real> Ls;
-  load_layers(R, reinterpret_cast<real*>(dyn_smem), Ls);
+  load_layers(R, reinterpret_cast<real*>(dyn_smem), Ls, threadIdx.x, blockDim.x);
+  __syncthreads();
   real* const er_out = rout->er;
   real* const et_out = rout->et;
   real* const hr_out = rout->hr;
@@ -73,7 +74,7 @@ __global__ void __launch_bounds__(256) fused_step_kernel(const Rec<real>* __rest
   const int4 p0 = __ldg(ft.patch + patch), p1 = __ldg(ft.patch + patch + 1);
   const int nhe = p1.x - p0.x, own_e = p0.y, nhf = p1.z - p0.z, own_f = p0.w;
   // the new H rows of the patch's halo, after the per-layer rows (16-byte aligned)
-  real* const s_ht = reinterpret_cast<real*>(dyn_smem) + (R.layer_reals + 3) / 4 * 4;
+  real* const s_ht = reinterpret_cast<real*>(dyn_smem) + R.layer_reals;
   real* const s_hr = s_ht + (size_t)nhe * Pn;
   // 1. new Ht (edges) and Hr (faces) from the old state
   for (int it = threadIdx.x; it < nhe * cn; it += blockDim.x) {
@@ -267,12 +268,11 @@ __global__ void __maxnreg__(kMaxRegs) kf_tma(const Rec<real>* __restrict__ rin, 
   __shared__ Rec<real> R;
   __shared__ __align__(8) uint64_t full[kMaxStages], empty[kMaxStages], group[kMaxStages];
   __shared__ int abort_flag;
-  Layers<real> Ls;
   Ring G;
   const int W = producers;
   if (threadIdx.x == 0)
     for (int s = 0; s < n_stages; ++s) mbar_init(group + s, (blockDim.x - 32 * W) / 32);  // made visible by ring_setup
-  ring_setup(R, rin, dyn_smem, full, empty, &abort_flag, stage_bytes, n_stages, COPY == 0 ? W : 32 * W, W, Ls, G);
+  ring_setup(R, rin, dyn_smem, full, empty, &abort_flag, stage_bytes, n_stages, COPY == 0 ? W : 32 * W, W, G);
   const int n = R.n_patches_e;
   const int p0 = (int)((long long)n * blockIdx.x / gridDim.x), p1 = (int)((long long)n * (blockIdx.x + 1) / gridDim.x);
   if (threadIdx.x < 32 * W) {
@@ -283,6 +283,8 @@ __global__ void __maxnreg__(kMaxRegs) kf_tma(const Rec<real>* __restrict__ rin, 
     real* const hr_out = rout->hr;
     real* const ht_out = rout->ht;
     const int ct = threadIdx.x - 32 * W, nct = blockDim.x - 32 * W;
+    Layers<real> Ls;
+    consumer_layers(R, dyn_smem, Ls, ct, nct);
     const real current = (R.n_src_er + R.n_src_et) > 0 ? (real)R.cur[istep] : real(0);
     consume_ring(G, p0, p1, [&](unsigned char* st, int s, uint32_t ph) {
       kf_consume<real, MAXDEG>(R, Ls, st, ct, nct, current, layout, group + s, ph, G, er_out, et_out, hr_out, ht_out);
@@ -314,9 +316,8 @@ __global__ void __maxnreg__(kMaxRegs) kf_tma_batch(const Rec<real>* __restrict__
     const int2 rg = rings[sg.x];
     batch_segment_start<real>(full, empty, group, prev, rg.y, (blockDim.x - 32 * W) / 32);
     prev = rg.y;
-    Layers<real> Ls;
     Ring G;
-    ring_setup(R, rin + sg.x, dyn_smem, full, empty, &abort_flag, rg.x, rg.y, COPY == 0 ? W : 32 * W, W, Ls, G);
+    ring_setup(R, rin + sg.x, dyn_smem, full, empty, &abort_flag, rg.x, rg.y, COPY == 0 ? W : 32 * W, W, G);
     if (threadIdx.x < 32 * W) {
       produce<COPY>(R, G, sg.y, sg.z, R.n_patches_e, R.dptr_e, R.desc_e, R.tab_e, threadIdx.x / 32, W);
     } else {
@@ -326,6 +327,8 @@ __global__ void __maxnreg__(kMaxRegs) kf_tma_batch(const Rec<real>* __restrict__
       real* const hr_out = ro->hr;
       real* const ht_out = ro->ht;
       const int ct = threadIdx.x - 32 * W, nct = blockDim.x - 32 * W;
+      Layers<real> Ls;
+      consumer_layers(R, dyn_smem, Ls, ct, nct);
       const real current = (R.n_src_er + R.n_src_et) > 0 ? (real)R.cur[istep] : real(0);
       consume_ring(G, sg.y, sg.z, [&](unsigned char* st, int s, uint32_t ph) {
         kf_consume<real, MAXDEG>(R, Ls, st, ct, nct, current, layout, group + s, ph, G, er_out, et_out, hr_out, ht_out);

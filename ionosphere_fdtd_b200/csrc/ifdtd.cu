@@ -1065,7 +1065,7 @@ int build_plan(ifdtd_plan* P, const ifdtd_mesh_desc* M, const ifdtd_grid_desc* G
       return owned_faces == (size_t)nF;  // every face written by exactly one patch
     };
     const int lreals = layer_reals(Pn, Pm, X->coef_rows_er != 1, 0, 0, 0, 0);
-    const size_t layer_bytes = (size_t)(lreals + 3) / 4 * 4 * sizeof(real);
+    const size_t layer_bytes = (size_t)lreals * sizeof(real);
     bool done = false;
     if (fused_staging != 1) {
       // the ring: the largest patch whose stage fits twice beside the per-layer rows
@@ -1156,22 +1156,16 @@ int build_plan(ifdtd_plan* P, const ifdtd_mesh_desc* M, const ifdtd_grid_desc* G
 
   // ---- radial metric rows, zero padded to Pn / Pm ----
   const double* r = G->radii_m;
-  std::vector<real> invr(Pn, 0), rr(Pn, 0), invcd(Pn, 0), mid(Pm, 0), invm(Pm, 0), invdr(Pm, 0);
+  std::vector<real> invr(Pn, 0), invm(Pm, 0);
   std::vector<double> m(L);
   for (int k = 0; k <= L; ++k) {
     if (!(r[k] > 0.0) || (k > 0 && !(r[k] > r[k - 1]))) return fail(IFDTD_ERR_ARGUMENT, "radii must increase");
     invr[k] = (real)(1.0 / r[k]);
-    rr[k] = (real)r[k];
   }
   for (int j = 0; j < L; ++j) {
     m[j] = 0.5 * (r[j] + r[j + 1]);
-    mid[j] = (real)m[j];
     invm[j] = (real)(1.0 / m[j]);
-    invdr[j] = (real)(1.0 / (r[j + 1] - r[j]));
   }
-  invcd[0] = (real)(2.0 / (r[1] - r[0]));
-  invcd[L] = (real)(2.0 / (r[L] - r[L - 1]));
-  for (int k = 1; k < L; ++k) invcd[k] = (real)(1.0 / (m[k] - m[k - 1]));
   // fused rows (float64 products, zero beyond the last node / midpoint):
   //   hA = dt/(mu0 r); hU, hD: weights of Et[k] and Et[k-1] in dt/mu0 (1/r) d(m Et)/dr
   //   (thin shell: d Et / dr) with zero (PEC-odd) ghosts; hC = dt/(mu0 m);
@@ -1247,27 +1241,14 @@ int build_plan(ifdtd_plan* P, const ifdtd_mesh_desc* M, const ifdtd_grid_desc* G
   UP(fe, face_e);
   UP(fv, face_v);
   UP(fw, face_w);
-  UP(invr, invr);
-  UP(rr, rr);
-  UP(mid, mid);
-  UP(invm, invm);
-  UP(invdr, invdr);
-  UP(invcd, invcd);
-  UP(hA, hA);
-  UP(hU, hU);
-  UP(hD, hD);
-  UP(hC, hC);
-  UP(vwl, vwl);
-  UP(vwu, vwu);
-  UP(eU, eU);
-  UP(eD, eD);
-  {
-    auto ca = pad_rows(X->ca_er, X->coef_rows_er, L + 1, Pn), cb = pad_rows(X->cb_er, X->coef_rows_er, L + 1, Pn);
-    auto ct = pad_rows(X->ca_et, X->coef_rows_et, L, Pm), cu = pad_rows(X->cb_et, X->coef_rows_et, L, Pm);
-    UP(ca, ca_er);
-    UP(cb, cb_er);
-    UP(ct, ca_et);
-    UP(cu, cb_et);
+  const bool coef_full = X->coef_rows_er != 1;
+  const auto ca_er = pad_rows(X->ca_er, X->coef_rows_er, L + 1, Pn), cb_er = pad_rows(X->cb_er, X->coef_rows_er, L + 1, Pn);
+  const auto ca_et = pad_rows(X->ca_et, X->coef_rows_et, L, Pm), cb_et = pad_rows(X->cb_et, X->coef_rows_et, L, Pm);
+  if (coef_full) {
+    UP(ca_er, ca_er);
+    UP(cb_er, cb_er);
+    UP(ca_et, ca_et);
+    UP(cb_et, cb_et);
   }
   {
     cudaError_t e1 = A.upload(fsign, &P->face_sign);
@@ -1282,18 +1263,18 @@ int build_plan(ifdtd_plan* P, const ifdtd_mesh_desc* M, const ifdtd_grid_desc* G
   P->face_e = R.face_e;
 
   // ---- surface impedance ----
+  std::vector<real> si_decay, si_drive, si_hist;
   P->T = X->si_terms;
   if (X->si_terms < 0 || X->si_terms > 256) return fail(IFDTD_ERR_ARGUMENT, "surface impedance terms out of range");
   if (X->si_terms > 0) {
     const int T = X->si_terms;
-    auto sc = cast<real>(X->si_scale, nE), dc = cast<real>(X->si_decay, T), dr = cast<real>(X->si_drive, T),
-         hw = cast<real>(X->si_history, T);
+    const auto sc = cast<real>(X->si_scale, nE);
+    si_decay = cast<real>(X->si_decay, T);
+    si_drive = cast<real>(X->si_drive, T);
+    si_hist = cast<real>(X->si_history, T);
     double hsum = 0.0;
     for (int p = 0; p < T; ++p) hsum += X->si_history[p];
     UP(sc, si_scale);
-    UP(dc, si_decay);
-    UP(dr, si_drive);
-    UP(hw, si_hist);
     R.si_metric = (real)X->si_metric;
     R.si_kappa = (real)(2.0 * G->time_step_s / (1.256637062120e-6 * (r[1] - r[0])));
     R.si_hist_sum = (real)hsum;
@@ -1301,6 +1282,8 @@ int build_plan(ifdtd_plan* P, const ifdtd_mesh_desc* M, const ifdtd_grid_desc* G
 
   // ---- plasma ----
   std::vector<real> pl, tn;  // (F, 12) reconstruction rows, (E, 8) edge tangents
+  std::vector<real> pc, bd;  // coefficients (S, 6, rows, Pm), unit B (rows, 3, Pm)
+  const bool plasma_full = X->plasma_rows == nF && nF != 1;
   P->S = X->plasma_species;
   if (X->plasma_species < 0 || X->plasma_species > IFDTD_MAX_SPECIES)
     return fail(IFDTD_ERR_ARGUMENT, "plasma species count out of range");
@@ -1346,16 +1329,16 @@ int build_plan(ifdtd_plan* P, const ifdtd_mesh_desc* M, const ifdtd_grid_desc* G
           tn[8 * (size_t)e + 4 + c] = (real)X->plasma_tangent_right[3 * (size_t)e + c];
         }
     }
-    auto pc = pad_rows(X->plasma_coef, S * 6 * rows, L, Pm);
+    pc = pad_rows(X->plasma_coef, S * 6 * rows, L, Pm);
     UP(pl, face_pl);
     UP(tn, tan);
-    UP(pc, pcoef);
+    if (plasma_full) UP(pc, pcoef);
     if (X->plasma_magnetized) {
-      std::vector<real> bd((size_t)rows * 3 * Pm, real(0));  // component-major (rows, 3, Pm)
+      bd.assign((size_t)rows * 3 * Pm, real(0));  // component-major
       for (int i = 0; i < rows; ++i)
         for (int j = 0; j < L; ++j)
           for (int c = 0; c < 3; ++c) bd[((size_t)i * 3 + c) * Pm + j] = (real)X->plasma_bdir[((size_t)i * L + j) * 3 + c];
-      UP(bd, bdir);
+      if (plasma_full) UP(bd, bdir);
     }
     if (S > 1) {
       cudaError_t e = A.alloc((size_t)nF * 3 * Pm * sizeof(real), &P->d_jtot);
@@ -1364,11 +1347,39 @@ int build_plan(ifdtd_plan* P, const ifdtd_mesh_desc* M, const ifdtd_grid_desc* G
     }
   }
 
+  // ---- per-layer rows: one block in the kernels' order ----
+  const int layer_n = layer_reals(Pn, Pm, coef_full, S, plasma_full, X->plasma_magnetized != 0, X->si_terms);
+  {
+    std::vector<real> block(layer_n, real(0));
+    Layers<real> at;
+    carve_layers(at, block.data(), Pn, Pm, coef_full, S, plasma_full, X->plasma_magnetized != 0, X->si_terms);
+    auto put = [](real* to, const std::vector<real>& row) {
+      if (to) std::copy(row.begin(), row.end(), to);
+    };
+    put(at.invr, invr);
+    put(at.hA, hA);
+    put(at.hU, hU);
+    put(at.hD, hD);
+    put(at.vwl, vwl);
+    put(at.vwu, vwu);
+    put(at.invm, invm);
+    put(at.hC, hC);
+    put(at.eU, eU);
+    put(at.eD, eD);
+    put(at.ca_er, ca_er);
+    put(at.cb_er, cb_er);
+    put(at.ca_et, ca_et);
+    put(at.cb_et, cb_et);
+    put(at.pc, pc);
+    put(at.bd, bd);
+    put(at.si_decay, si_decay);
+    put(at.si_drive, si_drive);
+    put(at.si_hist, si_hist);
+    UP(block, layers);
+  }
+
   // ---- pipelined kernels: copy descriptors and table blobs per patch ----
-  const int layer_block = pipe::layer_block_bytes(
-      layer_reals(Pn, Pm, X->coef_rows_er != 1, S, X->plasma_rows == nF && nF != 1, X->plasma_magnetized != 0,
-                  X->si_terms),
-      (int)sizeof(real));
+  const int layer_block = pipe::layer_block_bytes(layer_n, (int)sizeof(real));
   // static shared memory of the pipelined kernels: the record, 2 x 8 barriers
   // and the abort flag, well inside 1 KiB besides the record
   const int stage_budget = kSmemPerBlock - (int)sizeof(Rec<real>) - 1024 - layer_block;
@@ -1484,21 +1495,19 @@ int build_plan(ifdtd_plan* P, const ifdtd_mesh_desc* M, const ifdtd_grid_desc* G
   R.full = G->full_spherical ? 1 : 0;
   R.si_terms = X->si_terms;
   R.n_species = X->plasma_species;
-  R.plasma_full = X->plasma_rows == nF && nF != 1 ? 1 : 0;
+  R.plasma_full = plasma_full ? 1 : 0;
   R.magnetized = X->plasma_magnetized ? 1 : 0;
-  R.coef_full = X->coef_rows_er != 1 ? 1 : 0;
+  R.coef_full = coef_full ? 1 : 0;
   R.plasma_local = local ? 1 : 0;
   R.n_src_er = X->n_src_er;
   R.n_src_et = X->n_src_et;
   R.maxdeg = MD;
   R.slot_width = SW;
-  R.layer_reals = layer_reals(Pn, Pm, R.coef_full, X->plasma_species, R.plasma_full, R.magnetized, X->si_terms);
+  R.layer_reals = layer_n;
   P->smem_bytes = (size_t)R.layer_reals * sizeof(real);
   if (P->smem_bytes > 200 * 1024) return fail(IFDTD_ERR_UNSUPPORTED, "radial grid too fine for the shared per-layer rows");
   {
     // pipelined kernels: per-layer rows + n_stages ring stages in dynamic shared memory
-    if (pipe::layer_block_bytes(R.layer_reals, (int)sizeof(real)) != layer_block)
-      return fail(IFDTD_ERR_UNSUPPORTED, "inconsistent shared per-layer rows");
     auto stages = [&](bool ok, int stage) {
       return ok && stage > 0 ? std::min(pipe::kMaxStages, stage_budget / stage) : 0;
     };

@@ -495,11 +495,13 @@ __device__ __forceinline__ unsigned lane_pattern(int ct, int nct, int c, int lay
   return bits;
 }
 
-// Shared prologue: barriers, record, per-layer rows, this CTA's patch range.
+// Shared prologue: barriers, record and ring.  The per-layer rows are the
+// compute warps' own prologue (consumer_layers), so the producers' first copies
+// are on their way meanwhile.
 template <typename real>
 __device__ __forceinline__ void ring_setup(Rec<real>& R, const Rec<real>* recs, unsigned char* dyn, uint64_t* full,
                                            uint64_t* empty, int* abort_flag, int stage_bytes, int n_stages,
-                                           int full_arrivals, int producers, Layers<real>& Ls, Ring& G) {
+                                           int full_arrivals, int producers, Ring& G) {
   if (threadIdx.x == 0) {
     *abort_flag = 0;
     for (int s = 0; s < n_stages; ++s) {
@@ -509,7 +511,6 @@ __device__ __forceinline__ void ring_setup(Rec<real>& R, const Rec<real>* recs, 
     fence_mbar_init();
   }
   load_rec(R, recs);
-  load_layers(R, reinterpret_cast<real*>(dyn), Ls);
   G.stages = dyn + layer_block_bytes(R.layer_reals, (int)sizeof(real));
   G.stage_bytes = stage_bytes;
   G.n_stages = n_stages;
@@ -519,6 +520,18 @@ __device__ __forceinline__ void ring_setup(Rec<real>& R, const Rec<real>* recs, 
   G.status = R.status;
 }
 
+// The per-layer rows, copied by the compute threads (a barrier of the compute
+// warps alone).  Bound by latency: one block whose 16-byte loads are all in
+// flight together costs one trip to L2; copied row by row (up to 22 rows, each
+// waiting for the one before) the step took 23.5 instead of 16.2 us at s2 / 24
+// cells, 26.7 instead of 19.6 at s5 / 37 and 277 instead of 262 at s7 / 40.
+template <typename real>
+__device__ __forceinline__ void consumer_layers(const Rec<real>& R, unsigned char* dyn, Layers<real>& Ls, int ct,
+                                                int nct) {
+  load_layers(R, reinterpret_cast<real*>(dyn), Ls, ct, nct);
+  asm volatile("bar.sync 1, %0;" ::"r"(nct) : "memory");
+}
+
 template <typename real, bool PLASMA, int COPY>
 __global__ void __maxnreg__(kMaxRegs) kh_tma(const Rec<real>* __restrict__ recs, int stage_bytes, int n_stages,
                                              int producers, int layout) {
@@ -526,18 +539,19 @@ __global__ void __maxnreg__(kMaxRegs) kh_tma(const Rec<real>* __restrict__ recs,
   __shared__ Rec<real> R;
   __shared__ __align__(8) uint64_t full[kMaxStages], empty[kMaxStages], group[kMaxStages];
   __shared__ int abort_flag;
-  Layers<real> Ls;
   Ring G;
   const int W = producers;
   if (threadIdx.x == 0)
     for (int s = 0; s < n_stages; ++s) mbar_init(group + s, (blockDim.x - 32 * W) / 32);  // made visible by ring_setup
-  ring_setup(R, recs, dyn_smem, full, empty, &abort_flag, stage_bytes, n_stages, COPY == 0 ? W : 32 * W, W, Ls, G);
+  ring_setup(R, recs, dyn_smem, full, empty, &abort_flag, stage_bytes, n_stages, COPY == 0 ? W : 32 * W, W, G);
   const int n = R.n_patches_h;
   const int p0 = (int)((long long)n * blockIdx.x / gridDim.x), p1 = (int)((long long)n * (blockIdx.x + 1) / gridDim.x);
   if (threadIdx.x < 32 * W) {
     produce<COPY>(R, G, p0, p1, n, R.dptr_h, R.desc_h, R.tab_h, threadIdx.x / 32, W);
   } else {
     const int ct = threadIdx.x - 32 * W, nct = blockDim.x - 32 * W;
+    Layers<real> Ls;
+    consumer_layers(R, dyn_smem, Ls, ct, nct);
     consume_ring(G, p0, p1, [&](unsigned char* st, int s, uint32_t ph) {
       kh_consume<real, PLASMA>(R, Ls, st, ct, nct, group + s, ph, G, layout);
     });
@@ -551,16 +565,17 @@ __global__ void __maxnreg__(REGS) ke_tma(const Rec<real>* __restrict__ recs, int
   __shared__ Rec<real> R;
   __shared__ __align__(8) uint64_t full[kMaxStages], empty[kMaxStages];
   __shared__ int abort_flag;
-  Layers<real> Ls;
   Ring G;
   const int W = producers;
-  ring_setup(R, recs, dyn_smem, full, empty, &abort_flag, stage_bytes, n_stages, COPY == 0 ? W : 32 * W, W, Ls, G);
+  ring_setup(R, recs, dyn_smem, full, empty, &abort_flag, stage_bytes, n_stages, COPY == 0 ? W : 32 * W, W, G);
   const int n = R.n_patches_e;
   const int p0 = (int)((long long)n * blockIdx.x / gridDim.x), p1 = (int)((long long)n * (blockIdx.x + 1) / gridDim.x);
   if (threadIdx.x < 32 * W) {
     produce<COPY>(R, G, p0, p1, n, R.dptr_e, R.desc_e, R.tab_e, threadIdx.x / 32, W);
   } else {
     const int ct = threadIdx.x - 32 * W, nct = blockDim.x - 32 * W;
+    Layers<real> Ls;
+    consumer_layers(R, dyn_smem, Ls, ct, nct);
     const real current = (R.n_src_er + R.n_src_et) > 0 ? (real)R.cur[istep] : real(0);
     const unsigned pattern = lane_pattern(ct, nct, R.Pn / Lanes<real>::N, layout);
     consume_ring(G, p0, p1, [&](unsigned char* st, int s, uint32_t ph) {
@@ -610,13 +625,14 @@ __global__ void __maxnreg__(kMaxRegs) kh_tma_batch(const Rec<real>* __restrict__
     const int2 rg = rings[sg.x];
     batch_segment_start<real>(full, empty, group, prev, rg.y, (blockDim.x - 32 * W) / 32);
     prev = rg.y;
-    Layers<real> Ls;
     Ring G;
-    ring_setup(R, recs + sg.x, dyn_smem, full, empty, &abort_flag, rg.x, rg.y, COPY == 0 ? W : 32 * W, W, Ls, G);
+    ring_setup(R, recs + sg.x, dyn_smem, full, empty, &abort_flag, rg.x, rg.y, COPY == 0 ? W : 32 * W, W, G);
     if (threadIdx.x < 32 * W) {
       produce<COPY>(R, G, sg.y, sg.z, R.n_patches_h, R.dptr_h, R.desc_h, R.tab_h, threadIdx.x / 32, W);
     } else {
       const int ct = threadIdx.x - 32 * W, nct = blockDim.x - 32 * W;
+      Layers<real> Ls;
+      consumer_layers(R, dyn_smem, Ls, ct, nct);
       consume_ring(G, sg.y, sg.z, [&](unsigned char* st, int s, uint32_t ph) {
         kh_consume<real, PLASMA>(R, Ls, st, ct, nct, group + s, ph, G, layout);
       });
@@ -642,13 +658,14 @@ __global__ void __maxnreg__(REGS) ke_tma_batch(const Rec<real>* __restrict__ rec
     const int2 rg = rings[sg.x];
     batch_segment_start<real>(full, empty, group, prev, rg.y, (blockDim.x - 32 * W) / 32);
     prev = rg.y;
-    Layers<real> Ls;
     Ring G;
-    ring_setup(R, recs + sg.x, dyn_smem, full, empty, &abort_flag, rg.x, rg.y, COPY == 0 ? W : 32 * W, W, Ls, G);
+    ring_setup(R, recs + sg.x, dyn_smem, full, empty, &abort_flag, rg.x, rg.y, COPY == 0 ? W : 32 * W, W, G);
     if (threadIdx.x < 32 * W) {
       produce<COPY>(R, G, sg.y, sg.z, R.n_patches_e, R.dptr_e, R.desc_e, R.tab_e, threadIdx.x / 32, W);
     } else {
       const int ct = threadIdx.x - 32 * W, nct = blockDim.x - 32 * W;
+      Layers<real> Ls;
+      consumer_layers(R, dyn_smem, Ls, ct, nct);
       const real current = (R.n_src_er + R.n_src_et) > 0 ? (real)R.cur[istep] : real(0);
       const unsigned pattern = lane_pattern(ct, nct, R.Pn / Lanes<real>::N, layout);
       consume_ring(G, sg.y, sg.z, [&](unsigned char* st, int s, uint32_t ph) {

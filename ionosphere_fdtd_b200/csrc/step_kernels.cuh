@@ -80,21 +80,22 @@ struct Rec {
   const int *dptr_h, *dptr_e;
   const int4 *desc_h, *desc_e;
   const unsigned char *tab_h, *tab_e;
-  // radial metric rows (padded; staged in shared memory by the kernels)
-  const real *invr, *rr, *mid, *invm, *invdr, *invcd;
-  // fused per-layer rows: H-edge (hA, hU, hD), H-face (hC), E-vertex current
-  // weights (vwl, vwu), E-edge radial curl (eU, eD); zero beyond the grid
-  const real *hA, *hU, *hD, *hC, *vwl, *vwu, *eU, *eD;
+  // per-layer rows in the order of Layers (one block of layer_reals, padded to
+  // 16 bytes; staged in shared memory by the kernels): radial metric 1/r, 1/m and
+  // the fused rows H-edge (hA, hU, hD), E-vertex current weights (vwl, vwu),
+  // H-face (hC), E-edge radial curl (eU, eD), all zero beyond the grid; then the
+  // altitude-only coefficient rows
+  const real* layers;
   real dtmu;             // dt / mu0
-  // loss coefficients: (rows, Pn) / (rows, Pm), rows = 1 or V / E
+  // loss coefficients per entity, (V, Pn) / (E, Pm); null for altitude rows
   const real *ca_er, *cb_er, *ca_et, *cb_et;
   // sources (supports listed inline: the record lives in shared memory)
   int src_er_v[kMaxSources], src_er_k[kMaxSources], src_et_e[kMaxSources], src_et_j[kMaxSources];
   real src_er_c[kMaxSources], src_et_c[kMaxSources];
   // surface impedance
   real si_metric, si_kappa, si_hist_sum;
-  const real *si_scale, *si_decay, *si_drive, *si_hist;
-  // plasma: coefficients (S, 6, rows, Pm), unit B (rows, 3, Pm)
+  const real* si_scale;
+  // plasma per face: coefficients (S, 6, F, Pm), unit B (F, 3, Pm); null for altitude rows
   const real *pcoef, *bdir;
 };
 
@@ -187,21 +188,58 @@ __device__ __forceinline__ void st16(real* p, const Run<real>& r) {
 // Shared-memory view of the per-layer rows of one record.
 template <typename real>
 struct Layers {
-  real *invr, *rr, *invcd, *mid, *invm, *invdr;
+  real *invr, *invm;
   real *hA, *hU, *hD, *vwl, *vwu, *hC, *eU, *eD;
   real *ca_er, *cb_er, *ca_et, *cb_et;  // compressed coefficient rows (else null)
   real *pc, *bd;                        // compressed plasma rows (else null)
   real *si_decay, *si_drive, *si_hist;  // surface-impedance pole rows (else null)
 };
 
-// Number of reals of per-layer data staged in shared memory (host and device).
+// Number of reals of per-layer data staged in shared memory (host and device),
+// a whole number of 16-byte units.
 __host__ __device__ inline int layer_reals(int Pn, int Pm, int coef_full, int species, int plasma_full, int magnetized,
                                            int si_terms) {
-  int n = 8 * Pn + 6 * Pm;
+  int n = 6 * Pn + 4 * Pm;
   if (!coef_full) n += 2 * Pn + 2 * Pm;
   if (species > 0 && !plasma_full) n += 6 * species * Pm + (magnetized ? 3 * Pm : 0);
   n += 3 * si_terms;
-  return n;
+  return (n + 3) / 4 * 4;
+}
+
+// The rows' addresses inside a layer block at p (host packing and device view).
+template <typename real>
+__host__ __device__ __forceinline__ void carve_layers(Layers<real>& Ls, real* p, int Pn, int Pm, int coef_full,
+                                                      int species, int plasma_full, int magnetized, int si_terms) {
+  Ls.invr = p; p += Pn;
+  Ls.hA = p; p += Pn;
+  Ls.hU = p; p += Pn;
+  Ls.hD = p; p += Pn;
+  Ls.vwl = p; p += Pn;
+  Ls.vwu = p; p += Pn;
+  Ls.invm = p; p += Pm;
+  Ls.hC = p; p += Pm;
+  Ls.eU = p; p += Pm;
+  Ls.eD = p; p += Pm;
+  Ls.ca_er = Ls.cb_er = Ls.ca_et = Ls.cb_et = nullptr;
+  if (!coef_full) {
+    Ls.ca_er = p; p += Pn;
+    Ls.cb_er = p; p += Pn;
+    Ls.ca_et = p; p += Pm;
+    Ls.cb_et = p; p += Pm;
+  }
+  Ls.pc = Ls.bd = nullptr;
+  if (species > 0 && !plasma_full) {
+    Ls.pc = p; p += 6 * species * Pm;
+    if (magnetized) {
+      Ls.bd = p; p += 3 * Pm;
+    }
+  }
+  Ls.si_decay = Ls.si_drive = Ls.si_hist = nullptr;
+  if (si_terms > 0) {
+    Ls.si_decay = p; p += si_terms;
+    Ls.si_drive = p; p += si_terms;
+    Ls.si_hist = p;
+  }
 }
 
 // Copy the launch record into shared memory (one coalesced read per CTA).
@@ -215,74 +253,16 @@ __device__ __forceinline__ void load_rec(Rec<real>& dst, const Rec<real>* src) {
   __syncthreads();
 }
 
+// Copy the record's layer block to smem (16-byte aligned) with the n threads
+// t = 0 .. n - 1 and point Ls at its rows; the caller's barrier follows.  The
+// block is one run of 16-byte loads that are all in flight together.
 template <typename real>
-__device__ __forceinline__ void copy_row(real* dst, const real* src, int n) {
-  for (int i = threadIdx.x; i < n; i += blockDim.x) dst[i] = __ldg(src + i);
-}
-
-// Carve and fill the shared per-layer rows; ends with a barrier.
-template <typename real>
-__device__ __forceinline__ void load_layers(const Rec<real>& R, real* smem, Layers<real>& Ls) {
-  const int Pn = R.Pn, Pm = R.Pm;
-  real* p = smem;
-  Ls.invr = p; p += Pn;
-  Ls.rr = p; p += Pn;
-  Ls.invcd = p; p += Pn;
-  Ls.mid = p; p += Pm;
-  Ls.invm = p; p += Pm;
-  Ls.invdr = p; p += Pm;
-  copy_row(Ls.invr, R.invr, Pn);
-  copy_row(Ls.rr, R.rr, Pn);
-  copy_row(Ls.invcd, R.invcd, Pn);
-  copy_row(Ls.mid, R.mid, Pm);
-  copy_row(Ls.invm, R.invm, Pm);
-  copy_row(Ls.invdr, R.invdr, Pm);
-  Ls.hA = p; p += Pn;
-  Ls.hU = p; p += Pn;
-  Ls.hD = p; p += Pn;
-  Ls.vwl = p; p += Pn;
-  Ls.vwu = p; p += Pn;
-  Ls.hC = p; p += Pm;
-  Ls.eU = p; p += Pm;
-  Ls.eD = p; p += Pm;
-  copy_row(Ls.hA, R.hA, Pn);
-  copy_row(Ls.hU, R.hU, Pn);
-  copy_row(Ls.hD, R.hD, Pn);
-  copy_row(Ls.vwl, R.vwl, Pn);
-  copy_row(Ls.vwu, R.vwu, Pn);
-  copy_row(Ls.hC, R.hC, Pm);
-  copy_row(Ls.eU, R.eU, Pm);
-  copy_row(Ls.eD, R.eD, Pm);
-  Ls.ca_er = Ls.cb_er = Ls.ca_et = Ls.cb_et = nullptr;
-  if (!R.coef_full) {
-    Ls.ca_er = p; p += Pn;
-    Ls.cb_er = p; p += Pn;
-    Ls.ca_et = p; p += Pm;
-    Ls.cb_et = p; p += Pm;
-    copy_row(Ls.ca_er, R.ca_er, Pn);
-    copy_row(Ls.cb_er, R.cb_er, Pn);
-    copy_row(Ls.ca_et, R.ca_et, Pm);
-    copy_row(Ls.cb_et, R.cb_et, Pm);
-  }
-  Ls.pc = Ls.bd = nullptr;
-  if (R.n_species > 0 && !R.plasma_full) {
-    Ls.pc = p; p += 6 * R.n_species * Pm;
-    copy_row(Ls.pc, R.pcoef, 6 * R.n_species * Pm);
-    if (R.magnetized) {
-      Ls.bd = p; p += 3 * Pm;
-      copy_row(Ls.bd, R.bdir, 3 * Pm);
-    }
-  }
-  Ls.si_decay = Ls.si_drive = Ls.si_hist = nullptr;
-  if (R.si_terms > 0) {
-    Ls.si_decay = p; p += R.si_terms;
-    Ls.si_drive = p; p += R.si_terms;
-    Ls.si_hist = p; p += R.si_terms;
-    copy_row(Ls.si_decay, R.si_decay, R.si_terms);
-    copy_row(Ls.si_drive, R.si_drive, R.si_terms);
-    copy_row(Ls.si_hist, R.si_hist, R.si_terms);
-  }
-  __syncthreads();
+__device__ __forceinline__ void load_layers(const Rec<real>& R, real* smem, Layers<real>& Ls, int t, int n) {
+  const int units = R.layer_reals * (int)sizeof(real) / 16;
+  const uint4* src = reinterpret_cast<const uint4*>(R.layers);
+  uint4* dst = reinterpret_cast<uint4*>(smem);
+  for (int i = t; i < units; i += n) dst[i] = __ldg(src + i);
+  carve_layers(Ls, smem, R.Pn, R.Pm, R.coef_full, R.n_species, R.plasma_full, R.magnetized, R.si_terms);
 }
 
 // q = n / d for n < 2^24 and 1 <= d <= 1024 with m = ceil(2^32 / d); d = 1
@@ -893,7 +873,8 @@ __global__ void __launch_bounds__(256) kh_kernel(const Rec<real>* __restrict__ r
   member_patch(block_map, n_members, member, patch);
   load_rec(R, recs + member);
   Layers<real> Ls;
-  load_layers(R, reinterpret_cast<real*>(dyn_smem), Ls);
+  load_layers(R, reinterpret_cast<real*>(dyn_smem), Ls, threadIdx.x, blockDim.x);
+  __syncthreads();
   const int Pn = R.Pn, Pm = R.Pm, cn = Pn / N, cm = Pm / N;
   const uint32_t mag_cn = div_magic(cn), mag_cm = div_magic(cm);
   const int ea = R.eptr_h[patch], eb = R.eptr_h[patch + 1];
@@ -931,7 +912,8 @@ __global__ void __launch_bounds__(256) ke_kernel(const Rec<real>* __restrict__ r
   member_patch(block_map, n_members, member, patch);
   load_rec(R, recs + member);
   Layers<real> Ls;
-  load_layers(R, reinterpret_cast<real*>(dyn_smem), Ls);
+  load_layers(R, reinterpret_cast<real*>(dyn_smem), Ls, threadIdx.x, blockDim.x);
+  __syncthreads();
   const int Pn = R.Pn, Pm = R.Pm, SW = R.slot_width, cn = Pn / N, cm = Pm / N;
   const uint32_t mag_cn = div_magic(cn), mag_cm = div_magic(cm);
   const real current = (R.n_src_er + R.n_src_et) > 0 ? (real)R.cur[istep] : real(0);
