@@ -20,6 +20,7 @@ HEADERS = [
     PACKAGE / "csrc" / "step_kernels.cuh",
     PACKAGE / "csrc" / "pipe_kernels.cuh",
     PACKAGE / "csrc" / "fused_kernels.cuh",
+    PACKAGE / "csrc" / "loop_kernels.cuh",
     PACKAGE / "csrc" / "errors.cuh",
     ROOT / "include" / "ifdtd.h",
     ROOT / "include" / "ifdtd_surrogate.h",

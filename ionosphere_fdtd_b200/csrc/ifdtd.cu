@@ -16,6 +16,7 @@
 #include "../../include/ifdtd.h"
 #include "errors.cuh"
 #include "fused_kernels.cuh"
+#include "loop_kernels.cuh"
 #include "pipe_kernels.cuh"
 #include "step_kernels.cuh"
 
@@ -106,6 +107,8 @@ struct ifdtd_plan {
   int kh_stage = 0, ke_stage = 0, kh_stages = 0, ke_stages = 0, kh_grid = 0, ke_grid = 0, sm_count = 148;
   size_t smem_bytes = 0, kh_smem = 0, ke_smem = 0;
   int* d_status = nullptr;
+  bool loop = false;                         // many steps in one cooperative launch (kd_loop)
+  unsigned long long* d_arrivals = nullptr;  // its grid barrier
   bool plasma = false;
   bool plasma_local = false;     // the plasma current runs in face frames (converted around every call)
   const void* d_frame = nullptr;  // (F, 12) face-frame rows of those conversions
@@ -619,6 +622,18 @@ bool build_pipe_f(PipeTables& T, int n, const std::vector<int>& vptr, const std:
     if (T.tab.size() / 16 >= (size_t)1 << 31) return false;
   }
   return true;
+}
+
+// Runs of the larger phase, and the rounds a grid of one CTA per SM takes them in (kd_loop).
+template <typename real>
+int64_t loop_runs(const ifdtd_plan* P) {
+  const int64_t cn = P->Pn / Lanes<real>::N, cm = P->Pm / Lanes<real>::N;
+  return std::max(P->nE * cn + P->nF * cm, P->nV * cn + P->nE * cm);
+}
+template <typename real>
+int64_t loop_rounds(const ifdtd_plan* P) {
+  const int64_t once = (int64_t)P->sm_count * ((P->plasma ? kLoopThreads<real, true> : kLoopThreads<real, false>) - 32);
+  return (loop_runs<real>(P) + once - 1) / once;
 }
 
 template <typename real>
@@ -1546,6 +1561,29 @@ int build_plan(ifdtd_plan* P, const ifdtd_mesh_desc* M, const ifdtd_grid_desc* G
     R.status = (int*)st;
   }
   R.dtmu = (real)(G->time_step_s / 1.256637062120e-6);
+  // Steps in one cooperative launch while the whole grid takes a phase's runs in
+  // a few rounds and the launch geometry is automatic.  The line lies where it
+  // stops being faster than graph-replayed ring launches, us per step, loop
+  // against ring (no receivers, which cost the ring another 2-4 us):
+  //   s2 / 24 cells (0.05 rounds) 5.2 / 12.9; s5 / 37 (4.7) 13.2 / 17.9;
+  //   s6 / 20 (10.5) 22.4 / 27.0; s6 / 26 (13.2) 27.4 / 29.6; s6 / 34 (16.9) 36.7 / 34.4;
+  //   Drude plasma s5 / 40 (7.6) 21.0 / 26.0; magnetised s5 / 50 (9.4) 55.7 / 65.4;
+  //   float64 s5 / 30 (11.5) 17.9 / 19.9.
+  // With a surface impedance one thread walks an edge's poles, so the line lies
+  // lower: s4 / 31 (2.1 rounds) 7.6 / 15.1; plasma s5 / 20 (4.1) 19.4 / 22.4, s5 / 40
+  // (7.6) 29.2 / 29.1.
+  const bool auto_geometry =
+      !tune || (auto_h && auto_e && auto_threads && staging == 0 && !fused && e_threads_req == 0 && e_stages_req == 0 &&
+                (tune->producer_warps <= 0 || tune->producer_warps == 2) && tune->e_producer_warps <= 0 &&
+                e_copy_gap == 0 && lane_layout == 0);
+  if (auto_geometry && P->chunk > 0 && loop_rounds<real>(P) <= (X->si_terms > 0 ? 7 : 12)) {
+    P->loop = true;
+    void* at = nullptr;
+    cudaError_t e = A.alloc(sizeof(unsigned long long), &at);
+    if (e != cudaSuccess) return fail(IFDTD_ERR_CUDA, "allocation of the grid barrier failed");
+    CUDA_TRY(cudaMemset(at, 0, sizeof(unsigned long long)));
+    P->d_arrivals = (unsigned long long*)at;
+  }
   {
     void* cur = nullptr;
     cudaError_t e = A.alloc(std::max(P->chunk, 1) * sizeof(double), &cur);
@@ -1674,6 +1712,41 @@ cudaError_t launch_ke(ifdtd_plan* P, int istep, cudaStream_t st) {
   return P->plasma ? launch_ke_t<real, true, 12>(P, rec, istep, st) : launch_ke_t<real, false, 12>(P, rec, istep, st);
 }
 
+// Up to kLoopSteps leapfrog steps in one cooperative launch, one CTA per SM (a
+// bound on one launch's time, 1-7 ms; more steps per launch gain nothing).
+constexpr int kLoopSteps = 256;
+template <typename real, bool PL, int MD>
+cudaError_t launch_loop_t(ifdtd_plan* P, const LoopArgs& args, cudaStream_t st) {
+  auto k = kd_loop<real, PL, MD>;
+  cudaError_t e = allow_smem(k, P->smem_bytes);
+  if (e != cudaSuccess) return e;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(P->sm_count);
+  // just enough threads for the rounds the runs need, so that every CTA has its share
+  const int64_t per_sm = (loop_runs<real>(P) + P->sm_count - 1) / P->sm_count, rounds = loop_rounds<real>(P);
+  cfg.blockDim = dim3((unsigned)(((per_sm + rounds - 1) / rounds + 31) / 32 * 32 + 32));
+  cfg.dynamicSmemBytes = P->smem_bytes;
+  cfg.stream = st;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeCooperative;
+  at[0].val.cooperative = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, k, (const Rec<real>*)P->d_rec, args);
+}
+
+template <typename real>
+cudaError_t launch_loop(ifdtd_plan* P, const double* currents, int steps, const ifdtd_probe* probe, double* out,
+                        cudaStream_t st) {
+  LoopArgs a = {};
+  a.steps = steps;
+  a.currents = currents;
+  a.arrivals = P->d_arrivals;
+  if (probe) a.probe = {probe->kind, probe->rows, probe->width, probe->index, probe->layer, probe->weight, out};
+  if (P->maxdeg == 6) return P->plasma ? launch_loop_t<real, true, 6>(P, a, st) : launch_loop_t<real, false, 6>(P, a, st);
+  return P->plasma ? launch_loop_t<real, true, 12>(P, a, st) : launch_loop_t<real, false, 12>(P, a, st);
+}
+
 // One fused step: parity 0 reads the caller's arrays and writes the plan's
 // second copy, parity 1 the reverse.
 template <typename real>
@@ -1748,10 +1821,16 @@ int run_steps(ifdtd_plan* P, const ifdtd_state* st, const double* currents, int 
     explicit Range(const char* name) { nvtxRangePushA(name); }
     ~Range() { nvtxRangePop(); }
   } range(probe ? "ifdtd_step_sampled" : "ifdtd_step");
-  const int cap = std::max(P->chunk, 1);
+  const int cap = P->loop ? kLoopSteps : std::max(P->chunk, 1);
   int parity = 0;  // fused step: 1 while the state is in the plan's second copy
   for (int s0 = 0; s0 < n; s0 += cap) {
     const int c = std::min(cap, n - s0);
+    if (P->loop) {
+      double* out = probe ? out_rows + (size_t)s0 * probe->rows : nullptr;
+      const cudaError_t e = launch_loop<real>(P, currents ? currents + s0 : nullptr, c, probe, out, stream);
+      if (e != cudaSuccess) return fail(IFDTD_ERR_CUDA, std::string("step launch: ") + cudaGetErrorString(e));
+      continue;
+    }
     if (currents)
       CUDA_TRY(cudaMemcpyAsync(P->d_cur, currents + s0, c * sizeof(double), cudaMemcpyDeviceToDevice, stream));
     else
