@@ -247,6 +247,14 @@ int32_t ifdtd_sample(ifdtd_plan* plan, const ifdtd_state* state, const ifdtd_pro
  * (record_er_observations' inner loop, solver.py:1126-1135). */
 int32_t ifdtd_step_sampled(ifdtd_plan* plan, const ifdtd_state* state, const double* currents,
                            int32_t n_steps, const ifdtd_probe* probe, double* out_rows, void* stream);
+/* Step n_steps times, sampling n_probes (1 or 2) probes after every `every`
+ * steps and after the last one: sample s of probe q goes to row s of
+ * out_rows[q] (ceil(n_steps / every) rows).  record_h_observations' inner loop
+ * (solver.py:1206-1226).  currents, probes and output rows are read and written
+ * until the work enqueued on the stream is done. */
+int32_t ifdtd_step_recorded(ifdtd_plan* plan, const ifdtd_state* state, const double* currents,
+                            int32_t n_steps, int32_t every, int32_t n_probes, const ifdtd_probe* const* probes,
+                            double* const* out_rows, void* stream);
 
 /* Ensembles.  The reference runs an ensemble as a loop over GeodesicFDTD
  * objects, each calling step() / record_er_observations (solver.py:789-816,

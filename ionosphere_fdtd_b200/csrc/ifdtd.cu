@@ -79,16 +79,17 @@ struct DeviceArena {
 struct ifdtd_probe {
   ifdtd_plan* plan;
   int kind, rows, width;
-  int* index = nullptr;
-  int* layer = nullptr;
-  double* weight = nullptr;
-  double* staging = nullptr;  // (graph_chunk, rows)
-  DeviceArena arena;          // the probe's own device buffers
+  // one device block: weights, indices, layers
+  void* block = nullptr;
+  size_t bytes = 0;
+  const int* index = nullptr;
+  const int* layer = nullptr;
+  const double* weight = nullptr;
+  ~ifdtd_probe() { cudaFree(block); }
 };
 
 struct GraphEntry {
-  int chunk;
-  const ifdtd_probe* probe;
+  int chunk, blocks;  // steps, and blocks of each step's sampling launch (0: not sampled)
   cudaGraphExec_t exec;
 };
 
@@ -130,6 +131,14 @@ struct ifdtd_plan {
   cudaStream_t capture_stream = nullptr;
   std::vector<GraphEntry> graphs;
   std::vector<ifdtd_probe*> probes;
+  // the block of the probe destroyed last, for the next one (a recorded run
+  // makes and destroys its probes; at most kSpareBytes are kept)
+  void* spare = nullptr;
+  size_t spare_bytes = 0;
+  SampleSlot* d_slots = nullptr;  // the run's probes as the sampling launches read them
+  double* d_samples = nullptr;    // (graph_chunk, rows) of each slot
+  size_t sample_values = 0;
+  unsigned opted = 0;  // launch kinds whose shared-memory limit is raised
   std::vector<float> kh_cost, ke_cost;  // staged bytes per pipelined patch (balances batched launches)
   // fused step: halo tables, the record of the second field copy and its arrays
   bool fused = false;
@@ -145,10 +154,14 @@ struct ifdtd_plan {
   ~ifdtd_plan() {
     for (auto& g : graphs) cudaGraphExecDestroy(g.exec);
     if (capture_stream) cudaStreamDestroy(capture_stream);
+    cudaFree(spare);
+    cudaFree(d_samples);
   }
 };
 
 namespace {
+
+constexpr size_t kSpareBytes = (size_t)1 << 20;
 
 template <typename real>
 std::vector<real> cast(const double* p, size_t n) {
@@ -1591,6 +1604,12 @@ int build_plan(ifdtd_plan* P, const ifdtd_mesh_desc* M, const ifdtd_grid_desc* G
     P->d_cur = (double*)cur;
     R.cur = P->d_cur;
   }
+  {
+    void* slots = nullptr;
+    cudaError_t e = A.alloc(kMaxSlots * sizeof(SampleSlot), &slots);
+    if (e != cudaSuccess) return fail(IFDTD_ERR_CUDA, "allocation of the sample slots failed");
+    P->d_slots = (SampleSlot*)slots;
+  }
   P->h_rec.resize(sizeof(Rec<real>));
   std::memcpy(P->h_rec.data(), &R, sizeof(R));
   {
@@ -1648,6 +1667,16 @@ cudaError_t allow_smem(K kernel, size_t bytes) {
   return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
 }
 
+// allow_smem once per plan and launch kind (the query costs more than a launch).
+enum LaunchKind : unsigned { kLaunchKh = 1, kLaunchKe = 2, kLaunchKf = 4, kLaunchLoop = 8 };
+template <typename K>
+cudaError_t allow_smem_once(ifdtd_plan* P, LaunchKind kind, K kernel, size_t bytes) {
+  if (P->opted & kind) return cudaSuccess;
+  const cudaError_t e = allow_smem(kernel, bytes);
+  if (e == cudaSuccess) P->opted |= kind;
+  return e;
+}
+
 // Persistent grid: SM count x resident CTAs (from the occupancy calculator).
 template <typename K>
 cudaError_t persistent_grid(ifdtd_plan* P, K kernel, int threads, size_t smem, int n_patches, int* grid) {
@@ -1665,13 +1694,13 @@ cudaError_t launch_kh_t(ifdtd_plan* P, const Rec<real>* rec, cudaStream_t st) {
   if (P->h_mode == 2) {
     auto k = P->pipe_copy == 0 ? pipe::kh_tma<real, PL, 0> : pipe::kh_tma<real, PL, 1>;
     const int threads = P->threads + 32 * P->producers;
-    cudaError_t e = allow_smem(k, P->kh_smem);
+    cudaError_t e = allow_smem_once(P, kLaunchKh, k, P->kh_smem);
     if (e == cudaSuccess) e = persistent_grid(P, k, threads, P->kh_smem, P->n_patches, &P->kh_grid);
     if (e != cudaSuccess) return e;
     k<<<P->kh_grid, threads, P->kh_smem, st>>>(rec, P->kh_stage, P->kh_stages, P->producers, P->lanes);
   } else {
     auto k = kh_kernel<real, PL>;
-    cudaError_t e = allow_smem(k, P->smem_bytes);
+    cudaError_t e = allow_smem_once(P, kLaunchKh, k, P->smem_bytes);
     if (e != cudaSuccess) return e;
     k<<<P->n_patches, P->threads, P->smem_bytes, st>>>(rec, nullptr, 1);
   }
@@ -1685,13 +1714,13 @@ cudaError_t launch_ke_t(ifdtd_plan* P, const Rec<real>* rec, int istep, cudaStre
     auto k = threads > pipe::kMaxThreads ? pipe::ke_tma<real, PL, MD, 0, pipe::kWideRegs>
              : P->pipe_copy == 0         ? pipe::ke_tma<real, PL, MD, 0, pipe::kMaxRegs>
                                          : pipe::ke_tma<real, PL, MD, 1, pipe::kMaxRegs>;
-    cudaError_t e = allow_smem(k, P->ke_smem);
+    cudaError_t e = allow_smem_once(P, kLaunchKe, k, P->ke_smem);
     if (e == cudaSuccess) e = persistent_grid(P, k, threads, P->ke_smem, P->n_patches_e, &P->ke_grid);
     if (e != cudaSuccess) return e;
     k<<<P->ke_grid, threads, P->ke_smem, st>>>(rec, P->ke_stage, P->ke_stages, P->e_producers, istep, P->lanes);
   } else {
     auto k = ke_kernel<real, PL, MD>;
-    cudaError_t e = allow_smem(k, P->smem_bytes);
+    cudaError_t e = allow_smem_once(P, kLaunchKe, k, P->smem_bytes);
     if (e != cudaSuccess) return e;
     k<<<P->n_patches_e, P->threads, P->smem_bytes, st>>>(rec, nullptr, 1, istep);
   }
@@ -1718,7 +1747,7 @@ constexpr int kLoopSteps = 256;
 template <typename real, bool PL, int MD>
 cudaError_t launch_loop_t(ifdtd_plan* P, const LoopArgs& args, cudaStream_t st) {
   auto k = kd_loop<real, PL, MD>;
-  cudaError_t e = allow_smem(k, P->smem_bytes);
+  cudaError_t e = allow_smem_once(P, kLaunchLoop, k, P->smem_bytes);
   if (e != cudaSuccess) return e;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(P->sm_count);
@@ -1736,13 +1765,7 @@ cudaError_t launch_loop_t(ifdtd_plan* P, const LoopArgs& args, cudaStream_t st) 
 }
 
 template <typename real>
-cudaError_t launch_loop(ifdtd_plan* P, const double* currents, int steps, const ifdtd_probe* probe, double* out,
-                        cudaStream_t st) {
-  LoopArgs a = {};
-  a.steps = steps;
-  a.currents = currents;
-  a.arrivals = P->d_arrivals;
-  if (probe) a.probe = {probe->kind, probe->rows, probe->width, probe->index, probe->layer, probe->weight, out};
+cudaError_t launch_loop(ifdtd_plan* P, const LoopArgs& a, cudaStream_t st) {
   if (P->maxdeg == 6) return P->plasma ? launch_loop_t<real, true, 6>(P, a, st) : launch_loop_t<real, false, 6>(P, a, st);
   return P->plasma ? launch_loop_t<real, true, 12>(P, a, st) : launch_loop_t<real, false, 12>(P, a, st);
 }
@@ -1757,7 +1780,7 @@ cudaError_t launch_fused(ifdtd_plan* P, int istep, int parity, cudaStream_t st) 
     const int threads = P->kf_threads + 32 * P->kf_producers;
     auto k = P->maxdeg == 6 ? (P->pipe_copy == 0 ? pipe::kf_tma<real, 6, 0> : pipe::kf_tma<real, 6, 1>)
                             : (P->pipe_copy == 0 ? pipe::kf_tma<real, 12, 0> : pipe::kf_tma<real, 12, 1>);
-    cudaError_t e = allow_smem(k, P->kf_smem);
+    cudaError_t e = allow_smem_once(P, kLaunchKf, k, P->kf_smem);
     if (e == cudaSuccess) e = persistent_grid(P, k, threads, P->kf_smem, P->n_patches_e, &P->kf_grid);
     if (e != cudaSuccess) return e;
     k<<<P->kf_grid, threads, P->kf_smem, st>>>(parity ? b : a, parity ? a : b, P->kf_stage, P->kf_stages,
@@ -1765,14 +1788,15 @@ cudaError_t launch_fused(ifdtd_plan* P, int istep, int parity, cudaStream_t st) 
     return cudaGetLastError();
   }
   auto k = P->maxdeg == 6 ? fused_step_kernel<real, 6> : fused_step_kernel<real, 12>;
-  cudaError_t e = allow_smem(k, P->fused_smem);
+  cudaError_t e = allow_smem_once(P, kLaunchKf, k, P->fused_smem);
   if (e != cudaSuccess) return e;
   k<<<P->n_patches_e, P->threads, P->fused_smem, st>>>(parity ? b : a, parity ? a : b, P->fused_tab, istep);
   return cudaGetLastError();
 }
 
+// One step; with blocks > 0 its state is sampled into row `row` of the plan's slots.
 template <typename real>
-cudaError_t launch_step(ifdtd_plan* P, int istep, const ifdtd_probe* probe, int row, cudaStream_t st, int parity = 0) {
+cudaError_t launch_step(ifdtd_plan* P, int istep, int blocks, int row, cudaStream_t st, int parity = 0) {
   const Rec<real>* rec = (const Rec<real>*)P->d_rec;
   cudaError_t e;
   if (P->fused) {
@@ -1784,12 +1808,7 @@ cudaError_t launch_step(ifdtd_plan* P, int istep, const ifdtd_probe* probe, int 
     if (e == cudaSuccess) e = launch_ke<real>(P, istep, st);
   }
   if (e != cudaSuccess) return e;
-  if (probe) {
-    const int blocks = (probe->rows * 32 + 255) / 256;
-    sample_rec_kernel<real><<<blocks, 256, 0, st>>>(rec, probe->kind, probe->rows, probe->width, probe->index,
-                                                     probe->layer, probe->weight,
-                                                     probe->staging + (size_t)row * probe->rows);
-  }
+  if (blocks > 0) sample_slots_kernel<real><<<blocks, 256, 0, st>>>(rec, P->d_slots, row);
   return cudaGetLastError();
 }
 
@@ -1809,43 +1828,68 @@ cudaError_t plasma_frames(const ifdtd_plan* P, const ifdtd_state* st, int to_loc
   return cudaGetLastError();
 }
 
+// The probes of a recorded run: samples after every `every` steps and after the
+// last one, sample s of probe q in row s of out[q].
+struct Record {
+  int every = 1, n = 0;
+  const ifdtd_probe* probe[kMaxSlots] = {nullptr, nullptr};
+  double* out[kMaxSlots] = {nullptr, nullptr};
+  int rows() const {
+    int r = 0;
+    for (int q = 0; q < n; ++q) r += probe[q]->rows;
+    return r;
+  }
+};
+
+void fill_slot(SampleSlot& s, const ifdtd_probe* p, double* out) {
+  s = {p->kind, p->rows, p->width, p->index, p->layer, p->weight, out};
+}
+
+// Steps of a plan whose phases are launched (or replayed from graphs), `parity`
+// carried from call to call (fused step: 1 while the state is in the plan's
+// second copy); rec, if not null, is sampled after every step.
 template <typename real>
-int run_steps(ifdtd_plan* P, const ifdtd_state* st, const double* currents, int n, const ifdtd_probe* probe,
-              double* out_rows, cudaStream_t stream) {
-  int rc = bind_state<real>(P, st, stream);
-  if (rc) return rc;
-  if (n <= 0) return IFDTD_OK;
-  CUDA_TRY(plasma_frames<real>(P, st, 1, stream));
-  // NVTX range over the host-side enqueue of these steps (visible to profilers)
-  struct Range {
-    explicit Range(const char* name) { nvtxRangePushA(name); }
-    ~Range() { nvtxRangePop(); }
-  } range(probe ? "ifdtd_step_sampled" : "ifdtd_step");
-  const int cap = P->loop ? kLoopSteps : std::max(P->chunk, 1);
-  int parity = 0;  // fused step: 1 while the state is in the plan's second copy
+int run_launched(ifdtd_plan* P, const double* currents, int n, const Record* rec, int& parity, cudaStream_t stream) {
+  const int cap = std::max(P->chunk, 1);
+  // blocks of a sampling launch (8 rows each): powers of two, so a plan keeps few graphs
+  const int rows = rec ? rec->rows() : 0;
+  int blocks = rec ? 1 : 0;
+  while (blocks && blocks < 64 && 8 * blocks < rows) blocks *= 2;
+  size_t offset[kMaxSlots] = {0, 0};
+  if (rec) {
+    if ((size_t)cap * rows > P->sample_values) {
+      CUDA_TRY(cudaStreamSynchronize(stream));
+      cudaFree(P->d_samples);
+      P->d_samples = nullptr;
+      P->sample_values = 0;
+      CUDA_TRY(cudaMalloc((void**)&P->d_samples, (size_t)cap * rows * sizeof(double)));
+      P->sample_values = (size_t)cap * rows;
+    }
+    SampleSlot slots[kMaxSlots] = {};
+    for (int q = 0; q < rec->n; ++q) {
+      offset[q] = q ? (size_t)cap * rec->probe[0]->rows : 0;
+      fill_slot(slots[q], rec->probe[q], P->d_samples + offset[q]);
+    }
+    // pageable source: the runtime stages it before returning
+    CUDA_TRY(cudaMemcpyAsync(P->d_slots, slots, sizeof(slots), cudaMemcpyHostToDevice, stream));
+  }
   for (int s0 = 0; s0 < n; s0 += cap) {
     const int c = std::min(cap, n - s0);
-    if (P->loop) {
-      double* out = probe ? out_rows + (size_t)s0 * probe->rows : nullptr;
-      const cudaError_t e = launch_loop<real>(P, currents ? currents + s0 : nullptr, c, probe, out, stream);
-      if (e != cudaSuccess) return fail(IFDTD_ERR_CUDA, std::string("step launch: ") + cudaGetErrorString(e));
-      continue;
-    }
     if (currents)
       CUDA_TRY(cudaMemcpyAsync(P->d_cur, currents + s0, c * sizeof(double), cudaMemcpyDeviceToDevice, stream));
     else
       CUDA_TRY(cudaMemsetAsync(P->d_cur, 0, c * sizeof(double), stream));
-    if (P->chunk > 0 && c == P->chunk) {
+    if (P->chunk > 0 && c == P->chunk && !parity) {
       cudaGraphExec_t exec = nullptr;
       for (auto& g : P->graphs)
-        if (g.chunk == c && g.probe == probe) exec = g.exec;
+        if (g.chunk == c && g.blocks == blocks) exec = g.exec;
       if (!exec) {
         cudaGraph_t graph;
         CUDA_TRY(cudaStreamBeginCapture(P->capture_stream, cudaStreamCaptureModeThreadLocal));
         cudaError_t le = cudaSuccess;
         // an even chunk (fused plans) starts and ends in the caller's arrays
         for (int i = 0; i < c && le == cudaSuccess; ++i)
-          le = launch_step<real>(P, i, probe, i, P->capture_stream, P->fused ? (i & 1) : 0);
+          le = launch_step<real>(P, i, blocks, i, P->capture_stream, P->fused ? (i & 1) : 0);
         cudaError_t ce = cudaStreamEndCapture(P->capture_stream, &graph);
         if (le != cudaSuccess) {
           if (ce == cudaSuccess) cudaGraphDestroy(graph);  // the partial capture is not kept
@@ -1855,20 +1899,75 @@ int run_steps(ifdtd_plan* P, const ifdtd_state* st, const double* currents, int 
         cudaError_t ie = cudaGraphInstantiate(&exec, graph, 0);
         cudaGraphDestroy(graph);
         if (ie != cudaSuccess) return fail(IFDTD_ERR_CUDA, std::string("graph instantiate: ") + cudaGetErrorString(ie));
-        P->graphs.push_back({c, probe, exec});
+        P->graphs.push_back({c, blocks, exec});
       }
       CUDA_TRY(cudaGraphLaunch(exec, stream));
     } else {
       for (int i = 0; i < c; ++i) {
-        cudaError_t e = launch_step<real>(P, i, probe, i, stream, parity);
+        cudaError_t e = launch_step<real>(P, i, blocks, i, stream, parity);
         if (e != cudaSuccess) return fail(IFDTD_ERR_CUDA, std::string("step launch: ") + cudaGetErrorString(e));
         if (P->fused) parity ^= 1;
       }
     }
-    if (probe && out_rows)
-      CUDA_TRY(cudaMemcpyAsync(out_rows + (size_t)s0 * probe->rows, probe->staging,
-                               (size_t)c * probe->rows * sizeof(double), cudaMemcpyDeviceToDevice, stream));
+    if (rec)
+      for (int q = 0; q < rec->n; ++q) {
+        const size_t r = rec->probe[q]->rows;
+        CUDA_TRY(cudaMemcpyAsync(rec->out[q] + s0 * r, P->d_samples + offset[q], c * r * sizeof(double),
+                                 cudaMemcpyDeviceToDevice, stream));
+      }
   }
+  return IFDTD_OK;
+}
+
+// n steps of the loop kernel, sampled as rec says.
+template <typename real>
+int run_looped(ifdtd_plan* P, const double* currents, int n, const Record* rec, cudaStream_t stream) {
+  for (int s0 = 0; s0 < n; s0 += kLoopSteps) {
+    LoopArgs a = {};
+    a.steps = std::min(kLoopSteps, n - s0);
+    a.done = s0;
+    a.total = n;
+    a.every = rec ? rec->every : 1;
+    a.currents = currents ? currents + s0 : nullptr;
+    a.arrivals = P->d_arrivals;
+    for (int q = 0; rec && q < rec->n; ++q) fill_slot(a.slot[q], rec->probe[q], rec->out[q]);
+    const cudaError_t e = launch_loop<real>(P, a, stream);
+    if (e != cudaSuccess) return fail(IFDTD_ERR_CUDA, std::string("step launch: ") + cudaGetErrorString(e));
+  }
+  return IFDTD_OK;
+}
+
+template <typename real>
+int run_steps(ifdtd_plan* P, const ifdtd_state* st, const double* currents, int n, const Record* rec, cudaStream_t stream) {
+  int rc = bind_state<real>(P, st, stream);
+  if (rc) return rc;
+  if (n <= 0) return IFDTD_OK;
+  CUDA_TRY(plasma_frames<real>(P, st, 1, stream));
+  // NVTX range over the host-side enqueue of these steps (visible to profilers)
+  struct Range {
+    explicit Range(const char* name) { nvtxRangePushA(name); }
+    ~Range() { nvtxRangePop(); }
+  } range(rec ? "ifdtd_step_sampled" : "ifdtd_step");
+  int parity = 0;
+  if (P->loop) {
+    rc = run_looped<real>(P, currents, n, rec, stream);
+  } else if (!rec || rec->every == 1) {
+    rc = run_launched<real>(P, currents, n, rec, parity, stream);
+  } else {
+    // samples further apart than one step: the steps between them, then one sampling launch into the rows
+    for (int s0 = 0, k = 0; s0 < n && !rc; s0 += rec->every, ++k) {
+      const int c = std::min(rec->every, n - s0);
+      rc = run_launched<real>(P, currents ? currents + s0 : nullptr, c, nullptr, parity, stream);
+      if (rc) break;
+      SampleSlot slots[kMaxSlots] = {};
+      for (int q = 0; q < rec->n; ++q) fill_slot(slots[q], rec->probe[q], rec->out[q]);
+      if (k == 0) CUDA_TRY(cudaMemcpyAsync(P->d_slots, slots, sizeof(slots), cudaMemcpyHostToDevice, stream));
+      sample_slots_kernel<real><<<(rec->rows() + 7) / 8, 256, 0, stream>>>(
+          (const Rec<real>*)(parity ? P->d_rec_b : P->d_rec), P->d_slots, k);
+      CUDA_TRY(cudaGetLastError());
+    }
+  }
+  if (rc) return rc;
   if (parity) {
     // an odd number of fused steps ended in the second copy: move it to the caller's arrays
     void* const dst[4] = {st->er, st->et, st->hr, st->ht};
@@ -2481,8 +2580,8 @@ int32_t ifdtd_step(ifdtd_plan* plan, const ifdtd_state* state, const double* cur
   if (n_steps < 0) return fail(IFDTD_ERR_ARGUMENT, "negative step count");
   DeviceGuard guard(plan->device);
   cudaStream_t st = (cudaStream_t)stream;
-  return plan->dtype == 4 ? run_steps<float>(plan, state, currents, n_steps, nullptr, nullptr, st)
-                          : run_steps<double>(plan, state, currents, n_steps, nullptr, nullptr, st);
+  return plan->dtype == 4 ? run_steps<float>(plan, state, currents, n_steps, nullptr, st)
+                          : run_steps<double>(plan, state, currents, n_steps, nullptr, st);
 }
 
 int32_t ifdtd_update_magnetic(ifdtd_plan* plan, const ifdtd_state* state, void* stream) {
@@ -2581,12 +2680,15 @@ int32_t ifdtd_probe_create(ifdtd_plan* plan, int32_t field_kind, int32_t rows, i
   if (field_kind < 0 || field_kind > 3 || rows <= 0 || width <= 0) return fail(IFDTD_ERR_ARGUMENT, "bad probe shape");
   const int64_t n_ent = field_kind == 0 ? plan->nV : field_kind == 2 ? plan->nF : plan->nE;
   const int64_t n_lay = (field_kind == 0 || field_kind == 3) ? plan->L + 1 : plan->L;
-  const size_t n = (size_t)rows * width;
-  std::vector<int> idx(n), lay(n);
-  std::vector<double> w(weight, weight + n);
+  const size_t n = (size_t)rows * width, bytes = n * (sizeof(double) + 2 * sizeof(int));
+  std::vector<unsigned char> host(bytes);
+  double* const w = reinterpret_cast<double*>(host.data());
+  int* const idx = reinterpret_cast<int*>(w + n);
+  int* const lay = idx + n;
   for (size_t i = 0; i < n; ++i) {
     if (index[i] < 0 || index[i] >= n_ent || layer[i] < 0 || layer[i] >= n_lay)
       return fail(IFDTD_ERR_ARGUMENT, "probe index out of range");
+    w[i] = weight[i];
     idx[i] = (int)index[i];
     lay[i] = (int)layer[i];
   }
@@ -2596,41 +2698,39 @@ int32_t ifdtd_probe_create(ifdtd_plan* plan, int32_t field_kind, int32_t rows, i
   p->kind = field_kind;
   p->rows = rows;
   p->width = width;
-  const int* di = nullptr;
-  const int* dl = nullptr;
-  const double* dw = nullptr;
-  void* stg = nullptr;
-  if (p->arena.upload(idx, &di) != cudaSuccess || p->arena.upload(lay, &dl) != cudaSuccess ||
-      p->arena.upload(w, &dw) != cudaSuccess ||
-      p->arena.alloc((size_t)std::max(plan->chunk, 1) * rows * sizeof(double), &stg) != cudaSuccess) {
+  cudaError_t e = cudaSuccess;
+  if (plan->spare && plan->spare_bytes >= bytes) {
+    std::swap(p->block, plan->spare);
+    std::swap(p->bytes, plan->spare_bytes);
+  } else {
+    e = cudaMalloc(&p->block, bytes);
+    p->bytes = bytes;
+  }
+  if (e == cudaSuccess) e = cudaMemcpy(p->block, host.data(), bytes, cudaMemcpyHostToDevice);
+  if (e != cudaSuccess) {
     delete p;
     return fail(IFDTD_ERR_CUDA, "probe upload failed");
   }
-  p->index = (int*)di;
-  p->layer = (int*)dl;
-  p->weight = (double*)dw;
-  p->staging = (double*)stg;
+  p->weight = (const double*)p->block;
+  p->index = (const int*)(p->weight + n);
+  p->layer = p->index + n;
   plan->probes.push_back(p);
   *out = p;
   return IFDTD_OK;
 }
 
 int32_t ifdtd_probe_destroy(ifdtd_probe* probe) {
-  // the probe's buffers are released with it; graphs that sample it are dropped
+  // no launch may still read the probe's block when it is given back (or kept for the plan's next probe)
   if (!probe) return IFDTD_OK;
-  if (probe->plan) {
-    DeviceGuard guard(probe->plan->device);
+  ifdtd_plan* plan = probe->plan;
+  if (plan) {
+    DeviceGuard guard(plan->device);
     cudaDeviceSynchronize();
-    auto& v = probe->plan->probes;
+    auto& v = plan->probes;
     v.erase(std::remove(v.begin(), v.end(), probe), v.end());
-    auto& g = probe->plan->graphs;
-    for (auto it = g.begin(); it != g.end();) {
-      if (it->probe == probe) {
-        cudaGraphExecDestroy(it->exec);
-        it = g.erase(it);
-      } else {
-        ++it;
-      }
+    if (probe->bytes <= kSpareBytes && probe->bytes > plan->spare_bytes) {
+      std::swap(probe->block, plan->spare);
+      std::swap(probe->bytes, plan->spare_bytes);
     }
   }
   delete probe;
@@ -2659,12 +2759,27 @@ int32_t ifdtd_sample(ifdtd_plan* plan, const ifdtd_state* state, const ifdtd_pro
 
 int32_t ifdtd_step_sampled(ifdtd_plan* plan, const ifdtd_state* state, const double* currents, int32_t n_steps,
                            const ifdtd_probe* probe, double* out_rows, void* stream) {
-  if (!plan || !probe || !out_rows || probe->plan != plan) return fail(IFDTD_ERR_ARGUMENT, "bad sampled-step arguments");
+  return ifdtd_step_recorded(plan, state, currents, n_steps, 1, 1, &probe, &out_rows, stream);
+}
+
+int32_t ifdtd_step_recorded(ifdtd_plan* plan, const ifdtd_state* state, const double* currents, int32_t n_steps,
+                            int32_t every, int32_t n_probes, const ifdtd_probe* const* probes, double* const* out_rows,
+                            void* stream) {
+  if (!plan || !probes || !out_rows || n_probes < 1 || n_probes > kMaxSlots || every < 1)
+    return fail(IFDTD_ERR_ARGUMENT, "bad sampled-step arguments");
+  Record rec;
+  rec.every = every;
+  rec.n = n_probes;
+  for (int q = 0; q < n_probes; ++q) {
+    if (!probes[q] || !out_rows[q] || probes[q]->plan != plan) return fail(IFDTD_ERR_ARGUMENT, "bad sampled-step arguments");
+    rec.probe[q] = probes[q];
+    rec.out[q] = out_rows[q];
+  }
   if (n_steps < 0) return fail(IFDTD_ERR_ARGUMENT, "negative step count");
   DeviceGuard guard(plan->device);
   cudaStream_t st = (cudaStream_t)stream;
-  return plan->dtype == 4 ? run_steps<float>(plan, state, currents, n_steps, probe, out_rows, st)
-                          : run_steps<double>(plan, state, currents, n_steps, probe, out_rows, st);
+  return plan->dtype == 4 ? run_steps<float>(plan, state, currents, n_steps, &rec, st)
+                          : run_steps<double>(plan, state, currents, n_steps, &rec, st);
 }
 
 int32_t ifdtd_first_use_numbering(const int64_t* lo, const int64_t* hi, int64_t n, int64_t n_vertices, int64_t* rank,

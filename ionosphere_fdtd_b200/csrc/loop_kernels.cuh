@@ -29,42 +29,28 @@
 
 namespace ifdtd {
 
-struct LoopProbe {
-  int kind, rows, width;  // rows 0: nothing is sampled
-  const int* index;
-  const int* layer;
-  const double* weight;
-  double* out;  // (steps, rows)
-};
 struct LoopArgs {
-  int steps;
-  const double* currents;        // (steps) source current, or null
-  unsigned long long* arrivals;  // CTA arrivals so far: a multiple of the grid size between launches
-  LoopProbe probe;
+  int steps, done, total, every;  // this launch's steps, those before it in the run, the run's; steps per sample
+  const double* currents;         // (steps) source current, or null
+  unsigned long long* arrivals;   // CTA arrivals so far: a multiple of the grid size between launches
+  SampleSlot slot[kMaxSlots];
 };
 
 // Most threads of a CTA (one warp of them only samples).
 template <typename real, bool PLASMA>
 constexpr int kLoopThreads = sizeof(real) == 8 || PLASMA ? 512 : 768;
 
-// Rows blockIdx.x, blockIdx.x + gridDim.x, ... of one step's samples by one
-// warp; the arithmetic of sample_rec_kernel.  The fields are read past L1
-// (earlier phases of this launch wrote them).
+// This CTA's rows of the slots with E kinds (e) or H kinds, if the state after
+// the launch's step `step` is to be sampled; one warp.
 template <typename real>
-__device__ __forceinline__ void loop_sample(const Rec<real>& R, const LoopProbe& S, int step) {
-  const int lane = threadIdx.x & 31;
-  const real* field = S.kind == 0 ? R.er : S.kind == 1 ? R.et : S.kind == 2 ? R.hr : R.ht;
-  const int pitch = (S.kind == 0 || S.kind == 3) ? R.Pn : R.Pm;
-  for (int r = blockIdx.x; r < S.rows; r += gridDim.x) {
-    double acc = 0.0;
-    for (int q = lane; q < S.width; q += 32) {
-      const int o = r * S.width + q;
-      acc += __ldg(S.weight + o) * (double)__ldcg(field + (size_t)__ldg(S.index + o) * pitch + __ldg(S.layer + o));
-    }
+__device__ __forceinline__ void loop_sample(const Rec<real>& R, const LoopArgs& A, int step, bool e) {
+  const int n = A.done + step + 1;
+  if (n % A.every != 0 && n != A.total) return;
 #pragma unroll
-    for (int s = 16; s > 0; s >>= 1) acc += __shfl_down_sync(0xFFFFFFFFu, acc, s);
-    if (lane == 0) S.out[(size_t)step * S.rows + r] = acc;
-  }
+  for (int q = 0; q < kMaxSlots; ++q)
+    if ((A.slot[q].kind < 2) == e)
+      for (int r = blockIdx.x; r < A.slot[q].rows; r += gridDim.x)
+        sample_row(R, A.slot[q], r, (size_t)((n - 1) / A.every));
 }
 
 // Wait (bounded) until `arrivals` reaches target.
@@ -110,7 +96,11 @@ __global__ void __launch_bounds__(kLoopThreads<real, PLASMA>, 1)
   const int Pn = R.Pn, Pm = R.Pm, SW = R.slot_width, cn = Pn / N, cm = Pm / N;
   const uint32_t mag_cn = div_magic(cn), mag_cm = div_magic(cm);
   const real* Jsum = PLASMA ? jsum(R) : nullptr;
-  const bool sampling = A.probe.rows > 0, late = sampling && A.probe.kind < 2;
+  // whether Er / Et rows are sampled (after the E phase, by the next H phase) and Hr / Ht rows
+  bool late = false, early = false;
+#pragma unroll
+  for (int q = 0; q < kMaxSlots; ++q)
+    if (A.slot[q].rows > 0) (A.slot[q].kind < 2 ? late : early) = true;
   const bool sampler = threadIdx.x >= T;
   const int first = blockIdx.x * T + threadIdx.x, stride = gridDim.x * T;
   const int h_edges = R.nE * cn, h_runs = h_edges + R.nF * cm, e_verts = R.nV * cn, e_runs = e_verts + R.nE * cm;
@@ -166,7 +156,7 @@ __global__ void __launch_bounds__(kLoopThreads<real, PLASMA>, 1)
   bool ok = true;
   for (int step = 0; step < A.steps; ++step) {
     if (sampler) {
-      if (late && step > 0) loop_sample(R, A.probe, step - 1);
+      if (late && step > 0) loop_sample(R, A, step - 1, true);
     } else {
       for (int it = first; it < h_runs; it += stride) {
         const HRunTables t = ht;
@@ -189,7 +179,7 @@ __global__ void __launch_bounds__(kLoopThreads<real, PLASMA>, 1)
     ERunTables<MAXDEG> et = e_tables(first);
     if (!(ok = barrier())) break;
     if (sampler) {
-      if (sampling && !late) loop_sample(R, A.probe, step);
+      if (early) loop_sample(R, A, step, false);
     } else {
       const real current = A.currents && (R.n_src_er + R.n_src_et) > 0 ? (real)__ldg(A.currents + step) : real(0);
       for (int it = first; it < e_runs; it += stride) {
@@ -222,7 +212,7 @@ __global__ void __launch_bounds__(kLoopThreads<real, PLASMA>, 1)
     ht = h_tables(first);
     if ((step + 1 < A.steps || late) && !(ok = barrier())) break;
   }
-  if (ok && late && sampler) loop_sample(R, A.probe, A.steps - 1);
+  if (ok && late && sampler) loop_sample(R, A, A.steps - 1, true);
   if (threadIdx.x == 0 && arrived < barriers) atomicAdd(A.arrivals, (unsigned long long)(barriers - arrived));
 }
 

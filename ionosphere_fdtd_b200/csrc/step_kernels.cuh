@@ -1008,25 +1008,44 @@ __global__ void sample_kernel(const real* __restrict__ field, int pitch, int row
   if (lane == 0) out[warp] = acc;
 }
 
-// Probe of the field named by ``kind`` in the launch record (0 er, 1 et, 2 hr,
-// 3 ht): captured graphs read the current field pointer at run time.
+// One probe of a stepped run: field kind (0 er, 1 et, 2 hr, 3 ht), rows, support
+// width, the probe's device tables and the rows it writes.  rows 0: none.
+struct SampleSlot {
+  int kind, rows, width;
+  const int* index;
+  const int* layer;
+  const double* weight;
+  double* out;  // (samples, rows)
+};
+constexpr int kMaxSlots = 2;
+
+// Row r of the probe S: the weighted sum of its support points by one warp, in
+// the order of sample_kernel.  The fields are read past L1 (the loop kernel
+// writes them earlier in the same launch).
 template <typename real>
-__global__ void sample_rec_kernel(const Rec<real>* __restrict__ rec, int kind, int rows, int width,
-                                  const int* __restrict__ index, const int* __restrict__ layer,
-                                  const double* __restrict__ weight, double* __restrict__ out) {
-  const real* field = kind == 0 ? rec->er : kind == 1 ? rec->et : kind == 2 ? rec->hr : rec->ht;
-  const int pitch = (kind == 0 || kind == 3) ? rec->Pn : rec->Pm;
-  const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+__device__ __forceinline__ void sample_row(const Rec<real>& R, const SampleSlot& S, int r, size_t sample) {
   const int lane = threadIdx.x & 31;
-  if (warp >= rows) return;
+  const real* field = S.kind == 0 ? R.er : S.kind == 1 ? R.et : S.kind == 2 ? R.hr : R.ht;
+  const int pitch = (S.kind == 0 || S.kind == 3) ? R.Pn : R.Pm;
   double acc = 0.0;
-  for (int q = lane; q < width; q += 32) {
-    const int o = warp * width + q;
-    acc += weight[o] * (double)field[(size_t)index[o] * pitch + layer[o]];
+  for (int q = lane; q < S.width; q += 32) {
+    const int o = r * S.width + q;
+    acc += __ldg(S.weight + o) * (double)__ldcg(field + (size_t)__ldg(S.index + o) * pitch + __ldg(S.layer + o));
   }
 #pragma unroll
   for (int s = 16; s > 0; s >>= 1) acc += __shfl_down_sync(0xFFFFFFFFu, acc, s);
-  if (lane == 0) out[warp] = acc;
+  if (lane == 0) S.out[sample * S.rows + r] = acc;
+}
+
+// Every row of the slots in device memory: captured graphs name neither the
+// probes nor the fields, so one graph serves every recorded run of its plan.
+template <typename real>
+__global__ void sample_slots_kernel(const Rec<real>* __restrict__ rec, const SampleSlot* __restrict__ slots, int sample) {
+  const int warps = gridDim.x * (blockDim.x >> 5);
+  for (int w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; w < slots[0].rows + slots[1].rows; w += warps) {
+    const int first = slots[0].rows;
+    sample_row(*rec, slots[w < first ? 0 : 1], w < first ? w : w - first, (size_t)sample);
+  }
 }
 
 // One member's probe in a batched sampling launch: the member's record,

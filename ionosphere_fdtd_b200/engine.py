@@ -327,6 +327,22 @@ class Engine:
             "ifdtd_step_sampled",
         )
 
+    def step_recorded(self, state: N.State, currents: np.ndarray | None, count: int, every: int, probes, out_rows) -> None:
+        """``count`` steps, every probe sampled after each ``every`` steps and after the last one."""
+
+        if count <= 0:
+            return
+        cur = self._currents(currents, count)
+        n = len(probes)
+        N.check(
+            N.load().ifdtd_step_recorded(
+                self.plan, C.byref(state), None if cur is None else cur.data_ptr(), count, every, n,
+                (C.c_void_p * n)(*[p.handle.value for p in probes]), (C.c_void_p * n)(*[o.data_ptr() for o in out_rows]),
+                self.backend.stream_handle(),
+            ),
+            "ifdtd_step_recorded",
+        )
+
     def update_magnetic(self, state: N.State) -> None:
         N.check(N.load().ifdtd_update_magnetic(self.plan, C.byref(state), self.backend.stream_handle()), "ifdtd_update_magnetic")
 

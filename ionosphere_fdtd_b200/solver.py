@@ -13,6 +13,7 @@ constructor raises ``BackendUnavailableError``.
 
 from __future__ import annotations
 
+import math
 from dataclasses import dataclass
 from pathlib import Path
 from typing import Any
@@ -680,15 +681,17 @@ class GeodesicFDTD:
         p_hr = self._engine.probe("hr", faces, face_layers, fw)
         p_ht = self._engine.probe("ht", edges, edge_layers, ew)
         try:
-            start = self.steps
-            for row, target in enumerate(rows):
-                if row:
-                    self.step(int(target) - (self.steps - start))
-                state = self._state()
-                self._engine.sample(state, p_hr, hr_t[row])
-                self._engine.sample(state, p_ht, ht_t[row])
-                if int(target) % synchronize_every == 0:
-                    self.backend.synchronize()
+            state = self._state()
+            self._engine.sample(state, p_hr, hr_t[0])
+            self._engine.sample(state, p_ht, ht_t[0])
+            # the host waits where a sampled step is a multiple of synchronize_every
+            block = math.lcm(sample_every, synchronize_every)
+            for done in range(0, steps, block):
+                n, row = min(block, steps - done), 1 + done // sample_every
+                self._engine.step_recorded(state, self._source_currents(n), n, sample_every, (p_hr, p_ht), (hr_t[row:], ht_t[row:]))
+                self.steps += n
+                self.time_s = self.steps * self.time_step_s
+                self.backend.synchronize()
             self.backend.synchronize()
         finally:
             p_hr.close()

@@ -93,3 +93,30 @@ def test_loop_samples_every_field_kind(kind):
         probe.close()
     np.testing.assert_array_equal(rows[0], rows[1])
     assert np.abs(rows[0]).max() > 0.0
+
+
+@pytest.mark.parametrize("tuning", [dict(staging=2), dict(staging=2, graph_chunk=4), dict(fused_step=1)], ids=str)
+@pytest.mark.parametrize("steps,every", [(9, 1), (9, 2), (64, 7), (300, 128)])
+def test_recorded_h_samples_equal_single_steps(steps, every, tuning):
+    """One recorded run against stepping to each sample, on the loop and on the
+    launched plans (their sampled graph chunks and their steps between samples)."""
+
+    from ionosphere_fdtd_b200.engine import Tuning
+
+    case = CS.CASES["config1_s2"]
+    sims = [build_product(case, "float32"), build_product(case, "float32", tuning=Tuning(**tuning))]
+    rng = np.random.default_rng(4)
+    m, cells = sims[0].mesh, len(sims[0].radii_m) - 1
+    faces, edges = rng.integers(m.n_faces, size=(70, 1)), rng.integers(m.n_edges, size=(3, 2))
+    args = (faces, rng.integers(cells, size=(70, 1)), np.ones((70, 1)),
+            edges, rng.integers(cells + 1, size=(3, 2)), np.full((3, 2), 0.5))
+    single = build_product(case, "float32")
+    rows = [single.record_h_observations(*args, 0)]
+    while single.steps < steps:
+        single.step(min(every, steps - single.steps))
+        rows.append(single.record_h_observations(*args, 0))
+    for sim in sims:
+        for n, got in enumerate(sim.record_h_observations(*args, steps, sample_every=every)):
+            np.testing.assert_array_equal(got, np.concatenate([r[n] for r in rows]))
+        assert sim.steps == steps
+        _assert_same(sim, single)
