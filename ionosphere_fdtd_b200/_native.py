@@ -107,6 +107,23 @@ class State(C.Structure):
     ]
 
 
+class NetLayer(C.Structure):
+    """One layer of a surrogate network (``ifdtd_nn_layer``)."""
+
+    _fields_ = [(n, _i32) for n in ("fan_in", "fan_out", "act", "expand")] + [
+        (n, _vp) for n in ("w16", "bias", "z", "y", "dz", "dz16", "gw", "gb")]
+
+
+class NetParam(C.Structure):
+    """One parameter tensor of an Adam step (``ifdtd_nn_param``)."""
+
+    _fields_ = [(n, _vp) for n in ("w", "m", "v", "g", "w16")] + [("n", _i32)]
+
+
+NET_MAX_LAYERS = 32
+NET_TICKETS = 4096
+
+
 _SIGNATURES = {
     "ifdtd_version": ([], _i32),
     "ifdtd_last_error": ([C.c_char_p, C.c_size_t], _i32),
@@ -149,6 +166,10 @@ _SIGNATURES = {
     "ifdtd_nn_mse": ([_i32, _vp, _vp, _vp, _vp, _vp], _i32),
     "ifdtd_nn_wmse": ([_i32, _i32, _vp, _vp, _vp, _vp, _vp, _vp], _i32),
     "ifdtd_nn_adam": ([_i32, _vp, _vp, _vp, _vp, C.c_float, C.c_float, C.c_float, C.c_float, _i32, _vp, _vp], _i32),
+    "ifdtd_nn_forward": ([C.POINTER(NetLayer), _i32, _i32, _i32, _vp, _vp], _i32),
+    "ifdtd_nn_backward_bytes": ([C.POINTER(NetLayer), _i32, _i32, C.POINTER(C.c_int64)], _i32),
+    "ifdtd_nn_backward": ([C.POINTER(NetLayer), _i32, _i32, _vp, _vp, _vp, _vp, C.c_int64, _vp], _i32),
+    "ifdtd_nn_adam_all": ([C.POINTER(NetParam), _i32, C.c_float, C.c_float, C.c_float, C.c_float, _i32, _vp], _i32),
     "ifdtd_nn_to_bf16": ([C.c_int64, _vp, _vp, _vp], _i32),
     "ifdtd_edge_difference": ([_vp, _vp, _i32, _vp, _vp], _i32),
     "ifdtd_dual_edge_difference": ([_vp, _vp, _i32, _vp, _vp], _i32),

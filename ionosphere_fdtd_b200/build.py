@@ -15,13 +15,16 @@ from pathlib import Path
 
 PACKAGE = Path(__file__).resolve().parent
 ROOT = PACKAGE.parent
-SOURCES = [PACKAGE / "csrc" / "ifdtd.cu", PACKAGE / "csrc" / "surrogate.cu", PACKAGE / "csrc" / "gemm_tcgen05.cu"]
+SOURCES = [PACKAGE / "csrc" / "ifdtd.cu", PACKAGE / "csrc" / "surrogate.cu", PACKAGE / "csrc" / "gemm_tcgen05.cu",
+           PACKAGE / "csrc" / "surrogate_net.cu"]
 HEADERS = [
     PACKAGE / "csrc" / "step_kernels.cuh",
     PACKAGE / "csrc" / "pipe_kernels.cuh",
     PACKAGE / "csrc" / "fused_kernels.cuh",
     PACKAGE / "csrc" / "loop_kernels.cuh",
     PACKAGE / "csrc" / "errors.cuh",
+    PACKAGE / "csrc" / "silu.cuh",
+    PACKAGE / "csrc" / "tc_common.cuh",
     ROOT / "include" / "ifdtd.h",
     ROOT / "include" / "ifdtd_surrogate.h",
 ]

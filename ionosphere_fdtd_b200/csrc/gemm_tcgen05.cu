@@ -20,17 +20,12 @@
 // skips its remaining chunks and its epilogue, waits (again bounded) for the
 // MMAs it issued, frees its tensor memory and returns.  No operand is another
 // GPU's memory and no copy uses cluster multicast.
-#include <cuda.h>
-#include <cudaTypedefs.h>
-#include <cuda_bf16.h>
-#include <cuda_runtime.h>
-#include <stdint.h>
-
 #include <algorithm>
 #include <string>
 
 #include "../../include/ifdtd_surrogate.h"
 #include "errors.cuh"
+#include "tc_common.cuh"
 
 namespace ifdtd {
 namespace tc {
@@ -39,17 +34,13 @@ constexpr int TM = 128, TN = 128, TK = 64, THREADS = 128, STAGES = 2;
 constexpr int A_BYTES = TM * TK * 2, B_BYTES = TN * TK * 2, STAGE_BYTES = A_BYTES + B_BYTES;
 constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + 1024;  // + room to align the stages to 1024 bytes
 constexpr uint32_t TMEM_COLS = 128;
-constexpr uint64_t kWaitNs = 200ull * 1000 * 1000;
 
-__device__ int g_status;
 
 // Instruction descriptor of tcgen05.mma.kind::f16: fp32 accumulator (bits 4-5
 // = 1), A and B bf16 (bits 7-9 and 10-12 = 1), both K-major (bits 15, 16 = 0),
 // N >> 3 at bits 17-22, M >> 4 at bits 24-28; dense, no negation.
 constexpr uint32_t kInstrDesc =
     (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(TN >> 3) << 17) | ((uint32_t)(TM >> 4) << 24);
-
-__device__ __forceinline__ uint32_t smem_u32(const void* p) { return static_cast<uint32_t>(__cvta_generic_to_shared(p)); }
 
 // Shared-memory matrix descriptor: start address >> 4 (bits 0-13), leading
 // byte offset >> 4 (bits 16-29: the next core matrix along K, 128 B), stride
@@ -65,38 +56,6 @@ __device__ __forceinline__ uint64_t smem_desc(uint32_t addr) {
 __device__ __forceinline__ uint32_t core_offset(int row, int kg) {
   return (uint32_t)((((row >> 3) << 3) + kg) * 128 + ((row & 7) << 4));
 }
-
-__device__ __forceinline__ uint64_t global_ns() {
-  uint64_t t;
-  asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
-  return t;
-}
-
-__device__ __forceinline__ bool mbar_try(uint32_t bar, uint32_t parity) {
-  uint32_t ok;
-  asm volatile(
-      "{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}\n"
-      : "=r"(ok)
-      : "r"(bar), "r"(parity)
-      : "memory");
-  return ok != 0;
-}
-
-// Bounded wait for the phase of `bar` with this parity; false (and the status
-// bit set) when it did not complete within kWaitNs.
-__device__ __forceinline__ bool wait_bounded(uint32_t bar, uint32_t parity) {
-  if (mbar_try(bar, parity)) return true;
-  const uint64_t t0 = global_ns();
-  for (uint32_t i = 1; i < (1u << 30); ++i) {
-    if (mbar_try(bar, parity)) return true;
-    if ((i & 15u) == 0 && global_ns() - t0 > kWaitNs) break;
-  }
-  atomicOr(&g_status, 1);
-  return false;
-}
-
-__device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
-__device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
 
 // The 8 bf16 of op(X)[row][k0 .. k0 + 7] (zero outside rows x cols) as one
 // 16-byte piece.  op(X) is rows x cols: X row-major rows x cols (trans = 0,
@@ -275,6 +234,8 @@ int choose_splits(int tiles, int nk, size_t mn, size_t workspace_bytes) {
   return std::max(1, s);
 }
 
+cudaError_t net_status(int reset, int* out);  // surrogate_net.cu
+
 }  // namespace tc
 }  // namespace ifdtd
 
@@ -312,26 +273,6 @@ constexpr int XGROUP = 8;              // tile rasterisation: M-tiles per group
 constexpr uint32_t kInstrDescX =
     (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(XN >> 3) << 17) | ((uint32_t)(XM >> 4) << 24);
 
-// K-major operand with the 128-byte swizzle: rows of 128 bytes (64 bf16),
-// 8-row groups 1024 bytes apart (stride byte offset), the leading byte offset
-// unused (1), descriptor version 1, layout 2 (128-byte swizzle).  The K step of
-// 16 elements inside the 128-byte atom advances the start address by 32 bytes.
-__device__ __forceinline__ uint64_t smem_desc_sw128(uint32_t addr) {
-  return (uint64_t)((addr >> 4) & 0x3FFFu) | ((uint64_t)1 << 16) | ((uint64_t)(1024u >> 4) << 32) | ((uint64_t)1 << 46) |
-         ((uint64_t)2 << 61);
-}
-
-__device__ __forceinline__ void mbar_init_x(uint32_t bar, uint32_t count) {
-  asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(count) : "memory");
-}
-
-__device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap* map, int x, int y, uint32_t bar) {
-  asm volatile(
-      "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];" ::"r"(dst),
-      "l"(reinterpret_cast<uint64_t>(map)), "r"(x), "r"(y), "r"(bar)
-      : "memory");
-}
-
 // Output tile t of a tiles_m x tiles_n grid in grouped order: XGROUP M-tiles
 // sweep each N column together, so the CTAs running at once share B panels
 // (and A panels within a group) in L2.
@@ -346,10 +287,6 @@ __device__ __forceinline__ void tile_coords(int t, int tiles_m, int tiles_n, int
 
 __device__ __forceinline__ void mbar_arrive_x(uint32_t bar) {
   asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
-}
-
-__device__ __forceinline__ void tc_commit(uint32_t bar) {
-  asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
 }
 
 __global__ void __launch_bounds__(XTHREADS) gemm_tcgen05_tma(const __grid_constant__ CUtensorMap map_a,
@@ -492,25 +429,16 @@ __global__ void __launch_bounds__(XTHREADS) gemm_tcgen05_tma(const __grid_consta
   }
 }
 
-// 2-D tensor map of a row-major rows x K bf16 matrix with leading dimension
-// ld, boxes of box_rows x 64 with the 128-byte swizzle (zero fill outside).
-bool encode_kmajor(CUtensorMap* map, const void* base, int rows, int K, int ld, int box_rows) {
-  static PFN_cuTensorMapEncodeTiled encode = nullptr;
-  if (!encode) {
-    void* fn = nullptr;
-    cudaDriverEntryPointQueryResult q;
-    if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &fn, cudaEnableDefault, &q) != cudaSuccess ||
-        q != cudaDriverEntryPointSuccess || !fn)
-      return false;
-    encode = reinterpret_cast<PFN_cuTensorMapEncodeTiled>(fn);
-  }
-  const cuuint64_t dims[2] = {(cuuint64_t)K, (cuuint64_t)rows};
-  const cuuint64_t strides[1] = {(cuuint64_t)ld * 2};
-  const cuuint32_t box[2] = {(cuuint32_t)XK, (cuuint32_t)box_rows};
-  const cuuint32_t elem[2] = {1, 1};
-  return encode(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(base), dims, strides, box, elem,
-                CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-                CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+// Whether the TMA-fed kernel takes a product of K-major operands: enough output
+// tiles to spread over the SMs.
+bool tma_tiles(int m, int n) { return (size_t)((m + XM - 1) / XM) * ((n + XN - 1) / XN) >= 32; }
+
+// Splits of K that a product of the network takes (with kWorkspace bytes of
+// workspace): none on the TMA-fed kernel, which forward products may use.
+constexpr size_t kWorkspace = (size_t)16 << 20;
+int gemm_splits(int m, int n, int k, bool forward) {
+  if (forward && tma_tiles(m, n)) return 1;
+  return choose_splits(((m + TM - 1) / TM) * ((n + TN - 1) / TN), (k + TK - 1) / TK, (size_t)m * n, kWorkspace);
 }
 
 }  // namespace tc
@@ -535,9 +463,9 @@ int32_t ifdtd_nn_gemm_tc_ws(int32_t m, int32_t n, int32_t k, const void* a, int3
   // enough output tiles to spread over the SMs
   const bool kmajor = !trans_a && trans_b && lda % 8 == 0 && ldb % 8 == 0 && k % 8 == 0 &&
                       (reinterpret_cast<uintptr_t>(a) & 15) == 0 && (reinterpret_cast<uintptr_t>(b) & 15) == 0;
-  if (kmajor && (size_t)((m + XM - 1) / XM) * ((n + XN - 1) / XN) >= 32) {
+  if (kmajor && tma_tiles(m, n)) {
     CUtensorMap ma, mb;
-    if (encode_kmajor(&ma, a, m, k, lda, XM) && encode_kmajor(&mb, b, n, k, ldb, XN)) {
+    if (encode_rows(&ma, a, m, k, lda, XM) && encode_rows(&mb, b, n, k, ldb, XN)) {
       e = cudaFuncSetAttribute(gemm_tcgen05_tma, cudaFuncAttributeMaxDynamicSharedMemorySize, XSMEM);
       if (e != cudaSuccess)
         return ifdtd::record_error(IFDTD_ERR_CUDA, std::string("gemm_tcgen05_tma attribute: ") + cudaGetErrorString(e));
@@ -586,8 +514,10 @@ int32_t ifdtd_nn_gemm_tc_status(int32_t reset, int32_t* out) {
     const int zero = 0;
     e = cudaMemcpyToSymbol(g_status, &zero, sizeof(int));
   }
+  int net = 0;
+  if (e == cudaSuccess) e = net_status(reset, &net);
   if (e != cudaSuccess) return ifdtd::record_error(IFDTD_ERR_CUDA, std::string("gemm status: ") + cudaGetErrorString(e));
-  if (out) *out = v;
+  if (out) *out = v | net;
   return IFDTD_OK;
 }
 

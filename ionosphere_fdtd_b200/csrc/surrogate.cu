@@ -12,6 +12,7 @@
 
 #include "../../include/ifdtd_surrogate.h"
 #include "errors.cuh"
+#include "silu.cuh"
 
 namespace ifdtd {
 namespace nn {
@@ -100,12 +101,6 @@ __global__ void __launch_bounds__(THREADS) gemm_bf16(int M, int N, int K, const 
           *p = beta == 0.f ? v : v + beta * *p;
         }
       }
-}
-
-__device__ __forceinline__ float silu(float z) { return z / (1.f + expf(-z)); }
-__device__ __forceinline__ float silu_grad(float z) {
-  const float s = 1.f / (1.f + expf(-z));
-  return s * (1.f + z * (1.f - s));
 }
 
 // z += bias (per column); y = act(z) as bf16 (act 0: identity, 1: SiLU)

@@ -17,7 +17,9 @@ alternative (``gemm="mma"``).  Weights
 are FP32 masters with BF16 copies; activations between layers are BF16.
 Training uses the library's own kernels for every step (GEMMs, bias + SiLU,
 its derivative, bias sums, mean-squared error, Adam); PyTorch only holds the
-device buffers.
+device buffers.  The passes run as one launch per layer (``ifdtd_nn_forward``,
+``ifdtd_nn_backward``) where the network's rows are whole 16-byte units, else as
+one launch per step of every layer, with the same results bit for bit.
 
 The engine scores the surrogate and is its fallback: ``SurrogateEnsemble`` trains k
 networks from different seeds; a case whose members disagree by more than a
@@ -31,6 +33,7 @@ from dataclasses import dataclass, field
 import numpy as np
 
 from . import _native as N
+from .errors import BackendUnavailableError
 
 
 def _lib():
@@ -65,6 +68,7 @@ def architecture(inputs: int = 8, width: int = 512, depth: int = 4, samples: int
 
 
 GEMM_ENTRIES = {"tcgen05": "ifdtd_nn_gemm_tc_ws", "mma": "ifdtd_nn_gemm"}
+GROUP_ROWS = 4096  # cases per pass of a prediction (about 100 MB of bf16 activations)
 WORKSPACE_BYTES = 16 << 20  # split-K partial tiles of the tcgen05 GEMM
 
 
@@ -80,6 +84,7 @@ class TraceSurrogate:
         self.gemm_entry = GEMM_ENTRIES[gemm]
         self.torch = torch
         self._workspace = None
+        self._tickets = None
         self.device = torch.device(device)
         if self.device.type != "cuda":
             raise ValueError("the surrogate kernels run on a CUDA device")
@@ -96,6 +101,51 @@ class TraceSurrogate:
                 lst.append(torch.zeros(shape, dtype=torch.float32, device=self.device))
         self.step_count = 0
         self._acts: list = []
+        self._net = (N.NetLayer * len(layers))()
+        self._layout: tuple | None = None  # of the last batch size
+
+    # -- the last pass: activations (input, pre-activation per layer) and gradients.
+    # The one-launch-per-layer passes keep one block of each and cut it into tensors
+    # only when these are asked for.
+
+    @property
+    def _acts(self) -> list:
+        if self._acts_list is None:
+            (block, rows, at, x, out), self._acts_list = self._pass, []
+            for i, L in enumerate(self.layers):
+                last = i + 1 == len(self.layers)
+                z = out.view(rows[i], L.fan_out) if last else self._cut(block, at[2 * i], rows[i], L.fan_out, self.torch.float32)
+                self._acts_list.append((x, z))
+                if not last:
+                    x = self._cut(block, at[2 * i + 1], rows[i + 1], self.layers[i + 1].fan_in, self.torch.bfloat16)
+        return self._acts_list
+
+    @_acts.setter
+    def _acts(self, value: list) -> None:
+        self._acts_list, self._pass = value, None
+
+    def _gradients(self) -> tuple[list, list]:
+        if self._grad_lists is None:
+            if self._grad_block is None:
+                raise AttributeError("no gradients before a backward pass")
+            block, at = self._grad_block
+            n, f32 = len(self.layers), self.torch.float32
+            self._grad_lists = ([self._cut(block, at[i], L.fan_out, L.fan_in, f32) for i, L in enumerate(self.layers)],
+                                [self._cut(block, at[n + i], 1, L.fan_out, f32)[0] for i, L in enumerate(self.layers)])
+        return self._grad_lists
+
+    def _set_gradients(self, k: int, value: list) -> None:
+        lists = list(self._gradients() if self._grad_lists or self._grad_block else ([], []))
+        lists[k] = value
+        self._grad_lists, self._grad_block = tuple(lists), None
+
+    _grad_lists = _grad_block = _acts_list = _pass = None
+    gw = property(lambda self: self._gradients()[0], lambda self, v: self._set_gradients(0, v))
+    gb = property(lambda self: self._gradients()[1], lambda self, v: self._set_gradients(1, v))
+
+    @staticmethod
+    def _cut(block, offset: int, rows: int, cols: int, dtype):
+        return block[offset : offset + rows * cols * dtype.itemsize].view(dtype).view(rows, cols)
 
     def _stream(self) -> int:
         return int(self.torch.cuda.current_stream(self.device).cuda_stream)
@@ -114,6 +164,97 @@ class TraceSurrogate:
 
     def forward(self, x16):
         """x16: (B, inputs) bf16 device tensor -> (B, samples) fp32 predictions."""
+
+        return self._forward(x16, None)
+
+    def _whole_pass(self, x16) -> bool:
+        """Whether the one-launch-per-layer passes take this network and input: TMA
+        reads rows of whole 16-byte units."""
+
+        return (self.gemm_entry != "ifdtd_nn_gemm" and 0 < len(self.layers) <= N.NET_MAX_LAYERS and int(x16.shape[0]) > 0
+                and all(L.fan_in % 8 == 0 for L in self.layers) and x16.data_ptr() % 16 == 0)
+
+    def _bind_weights(self):
+        for d, L, w, b in zip(self._net, self.layers, self.w16, self.b):
+            d.fan_in, d.fan_out, d.act, d.expand = L.fan_in, L.fan_out, L.act, L.expand
+            d.w16, d.bias = w.data_ptr(), b.data_ptr()
+        return self._net
+
+    @staticmethod
+    def _offsets(sizes) -> tuple[list[int], int]:
+        """Byte offsets of arrays of these sizes in one block, on 256-byte boundaries, and the block's size."""
+
+        at, total = [], 0
+        for size in sizes:
+            at.append(total)
+            total += (size + 255) // 256 * 256
+        return at, total
+
+    def _batch_layout(self, batch: int) -> tuple:
+        """(batch, rows of every layer, outputs per case, forward offsets and bytes, backward scratch offsets and bytes)."""
+
+        if self._layout is None or self._layout[0] != batch:
+            rows = [batch]
+            for L in self.layers[:-1]:
+                rows.append(rows[-1] * L.expand)
+            forward = self._offsets([s * r * L.fan_out for r, L in zip(rows[:-1], self.layers) for s in (4, 2)])
+            need = N.C.c_int64()
+            _check(_lib().ifdtd_nn_backward_bytes(self._bind_weights(), len(rows), batch, N.C.byref(need)), "ifdtd_nn_backward_bytes")
+            work = int(need.value)
+            scratch = self._offsets([4 * r * L.fan_out for r, L in zip(rows, self.layers)]
+                                    + [2 * r * ((L.fan_out + 7) // 8 * 8) for r, L in zip(rows, self.layers)] + [work])
+            self._layout = (batch, rows, rows[-1] * self.layers[-1].fan_out // batch, forward, scratch, work)
+        return self._layout
+
+    def _block(self, size: int):
+        return self.torch.empty(size, dtype=self.torch.uint8, device=self.device)
+
+    def _forward(self, x16, out):
+        """Forward pass; ``out`` (contiguous fp32) receives the last layer's rows when given."""
+
+        if not self._whole_pass(x16):
+            z = self._forward_layers(x16)
+            return z if out is None else out.copy_(z)
+        batch, rows, samples, (at, size), _, _ = self._batch_layout(int(x16.shape[0]))
+        if out is None:
+            out = self.torch.empty((batch, samples), dtype=self.torch.float32, device=self.device)
+        block, net, n = self._block(size), self._bind_weights(), len(rows)
+        base = block.data_ptr()
+        for i in range(n - 1):
+            net[i].z, net[i].y = base + at[2 * i], base + at[2 * i + 1]
+        net[n - 1].z = out.data_ptr()
+        try:
+            _check(_lib().ifdtd_nn_forward(net, n, batch, batch, x16.data_ptr(), self._stream()), "ifdtd_nn_forward")
+        except BackendUnavailableError:
+            # a shape outside the whole-pass kernels' tiles
+            return out.copy_(self._forward_layers(x16))
+        self._acts_list, self._pass = None, (block, rows, at, x16, out)
+        return out
+
+    def _infer(self, x16, batch: int, out) -> bool:
+        """Several batches of ``batch`` rows in one pass that keeps no pre-activations."""
+
+        total = int(x16.shape[0])
+        if not self._whole_pass(x16):
+            return False
+        sizes, r = [], total
+        for L in self.layers[:-1]:
+            sizes.append(2 * r * L.fan_out)
+            r *= L.expand
+        at, size = self._offsets(sizes)
+        block, net, n = self._block(size), self._bind_weights(), len(self.layers)
+        base = block.data_ptr()
+        for i in range(n - 1):
+            net[i].z, net[i].y = None, base + at[i]
+        net[n - 1].z = out.data_ptr()
+        try:
+            _check(_lib().ifdtd_nn_forward(net, n, total, batch, x16.data_ptr(), self._stream()), "ifdtd_nn_forward")
+        except BackendUnavailableError:
+            return False
+        return True
+
+    def _forward_layers(self, x16):
+        """The same pass, one product and one activation launch per layer."""
 
         torch = self.torch
         lib, s = _lib(), self._stream()
@@ -137,9 +278,42 @@ class TraceSurrogate:
     def backward(self, grad):
         """Gradients of every weight and bias from dLoss/dpred (B, samples) fp32."""
 
+        if self._pass is not None and self._backward_whole(grad):
+            return
+        self._backward_layers(grad)
+
+    def _backward_whole(self, grad) -> bool:
+        torch, n = self.torch, len(self.layers)
+        block, rows, zy, x, out = self._pass
+        dy = grad.reshape(rows[-1], self.layers[-1].fan_out).contiguous()
+        if dy.data_ptr() % 16:
+            dy = dy.clone()
+        _, _, _, _, (at, size), work = self._batch_layout(rows[0])
+        scratch, gat = self._block(size), self._offsets([4 * L.fan_out * L.fan_in for L in self.layers] + [4 * L.fan_out for L in self.layers])
+        grads, net = self._block(gat[1]), self._bind_weights()
+        base, sbase, gbase = block.data_ptr(), scratch.data_ptr(), grads.data_ptr()
+        for i, d in enumerate(net):
+            if i + 1 < n:
+                d.z, d.y = base + zy[2 * i], base + zy[2 * i + 1]
+            else:
+                d.z = out.data_ptr()
+            d.dz, d.dz16, d.gw, d.gb = sbase + at[i], sbase + at[n + i], gbase + gat[0][i], gbase + gat[0][n + i]
+        if self._tickets is None:
+            self._tickets = torch.zeros(N.NET_TICKETS, dtype=torch.int32, device=self.device)
+        try:
+            _check(_lib().ifdtd_nn_backward(net, n, rows[0], x.data_ptr(), dy.data_ptr(), self._tickets.data_ptr(), sbase + at[2 * n], work,
+                                            self._stream()), "ifdtd_nn_backward")
+        except BackendUnavailableError:
+            return False  # a shape outside the whole-pass kernels' tiles
+        self._grad_lists, self._grad_block = None, (grads, gat[0])
+        return True
+
+    def _backward_layers(self, grad):
+        """The same gradients, one launch per step of every layer."""
+
         torch = self.torch
         lib, s = _lib(), self._stream()
-        self.gw, self.gb = [None] * len(self.layers), [None] * len(self.layers)
+        self._grad_block, self._grad_lists = None, ([None] * len(self.layers), [None] * len(self.layers))
         dy = grad.reshape(self._acts[-1][1].shape).contiguous()
         for i in range(len(self.layers) - 1, -1, -1):
             L = self.layers[i]
@@ -181,13 +355,21 @@ class TraceSurrogate:
         return loss, grad
 
     def adam_step(self, lr: float, beta1: float = 0.9, beta2: float = 0.999, eps: float = 1e-8) -> None:
-        lib, s = _lib(), self._stream()
+        n = len(self.layers)
+        if self._grad_lists is None and self._grad_block is not None:
+            base = self._grad_block[0].data_ptr()
+            grads = [base + at for at in self._grad_block[1]]
+        else:
+            grads = [g.data_ptr() for g in self.gw + self.gb]
         self.step_count += 1
-        for i in range(len(self.layers)):
-            _check(lib.ifdtd_nn_adam(int(self.w[i].numel()), self.w[i].data_ptr(), self.gw[i].data_ptr(), self.mw[i].data_ptr(),
-                                     self.vw[i].data_ptr(), lr, beta1, beta2, eps, self.step_count, self.w16[i].data_ptr(), s), "ifdtd_nn_adam")
-            _check(lib.ifdtd_nn_adam(int(self.b[i].numel()), self.b[i].data_ptr(), self.gb[i].data_ptr(), self.mb[i].data_ptr(),
-                                     self.vb[i].data_ptr(), lr, beta1, beta2, eps, self.step_count, None, s), "ifdtd_nn_adam")
+        params = [(w.data_ptr(), m.data_ptr(), v.data_ptr(), grads[i], w16.data_ptr(), w.numel())
+                  for i, (w, m, v, w16) in enumerate(zip(self.w, self.mw, self.vw, self.w16))]
+        params += [(b.data_ptr(), m.data_ptr(), v.data_ptr(), grads[n + i], None, b.numel())
+                   for i, (b, m, v) in enumerate(zip(self.b, self.mb, self.vb))]
+        for k in range(0, len(params), 64):
+            part = params[k : k + 64]
+            _check(_lib().ifdtd_nn_adam_all((N.NetParam * len(part))(*part), len(part), lr, beta1, beta2, eps, self.step_count, self._stream()),
+                   "ifdtd_nn_adam_all")
 
     def fit(self, x, y, *, iterations: int, batch: int, lr: float = 1e-3, seed: int = 0, lr_final: float | None = None,
             relative: bool = False) -> list[float]:
@@ -219,9 +401,25 @@ class TraceSurrogate:
         return [float(v) for v in torch.cat(losses).cpu()]
 
     def predict(self, x, batch: int = 512):
-        torch = self.torch
-        out = [self.forward(x[i : i + batch].contiguous()).clone() for i in range(0, int(x.shape[0]), batch)]
-        return torch.cat(out)
+        torch, rows = self.torch, int(x.shape[0])
+        if not range(0, rows, batch):
+            return torch.cat([])  # refused by torch: there is nothing to predict
+        samples = self.layers[-1].fan_out
+        for L in self.layers[:-1]:
+            samples *= L.expand
+        out = torch.empty((rows, samples), dtype=torch.float32, device=self.device)
+        # the batches but the last in groups of several per pass, the last as a plain
+        # forward pass (its activations stay for a backward pass)
+        group = batch * max(1, GROUP_ROWS // batch)
+        i, last = 0, (rows - 1) // batch * batch
+        while i < last:
+            n = min(group, last - i)
+            if not self._infer(x[i : i + n].contiguous(), batch, out[i : i + n]):
+                n = batch
+                self._forward(x[i : i + n].contiguous(), out[i : i + n])
+            i += n
+        self._forward(x[last:].contiguous(), out[last:])
+        return out
 
 
 @dataclass
