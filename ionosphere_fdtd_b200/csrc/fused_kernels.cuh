@@ -276,7 +276,7 @@ __global__ void __maxnreg__(kMaxRegs) kf_tma(const Rec<real>* __restrict__ rin, 
   const int n = R.n_patches_e;
   const int p0 = (int)((long long)n * blockIdx.x / gridDim.x), p1 = (int)((long long)n * (blockIdx.x + 1) / gridDim.x);
   if (threadIdx.x < 32 * W) {
-    produce<COPY>(R, G, p0, p1, n, R.dptr_e, R.desc_e, R.tab_e, threadIdx.x / 32, W);
+    produce<COPY>(R, G, p0, p1, n, R.dptr_e, R.desc_e, threadIdx.x / 32, W);
   } else {
     real* const er_out = rout->er;
     real* const et_out = rout->et;
@@ -319,7 +319,7 @@ __global__ void __maxnreg__(kMaxRegs) kf_tma_batch(const Rec<real>* __restrict__
     Ring G;
     ring_setup(R, rin + sg.x, dyn_smem, full, empty, &abort_flag, rg.x, rg.y, COPY == 0 ? W : 32 * W, W, G);
     if (threadIdx.x < 32 * W) {
-      produce<COPY>(R, G, sg.y, sg.z, R.n_patches_e, R.dptr_e, R.desc_e, R.tab_e, threadIdx.x / 32, W);
+      produce<COPY>(R, G, sg.y, sg.z, R.n_patches_e, R.dptr_e, R.desc_e, threadIdx.x / 32, W);
     } else {
       const Rec<real>* ro = rout + sg.x;
       real* const er_out = ro->er;

@@ -236,34 +236,46 @@ void add_runs(std::vector<int4>& desc, int src, const std::vector<std::pair<int,
 
 int round128(int n) { return (n + 127) / 128 * 128; }
 
+// Row bytes and rows of a copy source.
+struct SourceShape {
+  int rb, Pn, Pm, Tsi, nV, nE, nF, S;
+  bool of(int src, long tab_units, long& row, long& rows) const {
+    using namespace pipe;
+    switch (src) {
+      case kSrcEr: row = Pn * rb; rows = nV; break;
+      case kSrcEt: row = Pm * rb; rows = nE; break;
+      case kSrcHt: row = Pn * rb; rows = nE; break;
+      case kSrcHr: row = Pm * rb; rows = nF; break;
+      case kSrcJsum: row = 3 * Pm * rb; rows = S > 0 ? nF : 0; break;
+      case kSrcSi: row = Tsi * rb; rows = Tsi > 0 ? nE : 0; break;
+      case kSrcTabH:
+      case kSrcTabE: row = 16; rows = tab_units; break;
+      default:
+        if (src < kSrcJ0 || src >= kSrcJ0 + S) return false;
+        row = 3 * Pm * rb;
+        rows = nF;
+    }
+    return row > 0;
+  }
+};
+
 // Check every copy descriptor before upload: a positive multiple of 16 bytes
 // of whole rows, a 16-byte aligned destination inside the patch's stage, source
-// rows inside their array, the blob first and inside the table, and at most
-// 2^20 - 1 bytes per patch (the mbarrier transaction limit).
-bool descriptors_valid(const PipeTables& T, int rb, int Pn, int Pm, int Tsi, int nV, int nE, int nF, int S) {
-  using namespace pipe;
+// rows inside their array, the blob (source `tab`) first and inside the table, and
+// at most 2^20 - 1 bytes per patch (the mbarrier transaction limit).  Then turn
+// the first rows into offsets in 16-byte units, as the copies read them.
+bool finish_descriptors(PipeTables& T, int tab, const SourceShape& shape) {
   for (size_t q = 0; q + 1 < T.dptr.size(); ++q) {
     long total = 0;
     for (int d = T.dptr[q]; d < T.dptr[q + 1]; ++d) {
-      const int4 x = T.desc[d];
-      int row = 0;
-      long rows = 0;
-      switch (x.x) {
-        case kSrcEr: row = Pn * rb; rows = nV; break;
-        case kSrcEt: row = Pm * rb; rows = nE; break;
-        case kSrcHt: row = Pn * rb; rows = nE; break;
-        case kSrcHr: row = Pm * rb; rows = nF; break;
-        case kSrcJsum: row = 3 * Pm * rb; rows = S > 0 ? nF : 0; break;
-        case kSrcSi: row = Tsi * rb; rows = Tsi > 0 ? nE : 0; break;
-        case kSrcTab: row = 16; rows = (long)(T.tab.size() / 16); break;
-        default:
-          if (x.x < kSrcJ0 || x.x >= kSrcJ0 + S) return false;
-          row = 3 * Pm * rb;
-          rows = nF;
-      }
-      if (row <= 0 || x.w <= 0 || x.w % 16 || x.w % row || x.z % 16 || x.z < 0 || x.z + x.w > T.stage_bytes) return false;
+      int4& x = T.desc[d];
+      long row = 0, rows = 0;
+      if (!shape.of(x.x, (long)(T.tab.size() / 16), row, rows)) return false;
+      if (x.w <= 0 || x.w % 16 || x.w % row || x.z % 16 || x.z < 0 || x.z + x.w > T.stage_bytes) return false;
       if (x.y < 0 || (long)x.y + x.w / row > rows) return false;
-      if ((x.x == kSrcTab) != (d == T.dptr[q]) || (x.x == kSrcTab && x.z != 0)) return false;
+      if ((x.x == tab) != (d == T.dptr[q]) || (x.x == tab && x.z != 0)) return false;
+      if (row % 16 || x.y * (row / 16) >= 1L << 32) return false;
+      x.y = (int)(uint32_t)(x.y * (row / 16));
       total += x.w;
     }
     if (total >= (1 << 20)) return false;
@@ -324,13 +336,13 @@ bool build_pipe_h(PipeTables& T, int n, int fpp, int nF, const std::vector<int>&
     eloc.resize(ne);
     for (int el = 0; el < ne; ++el) {
       const int e = ea + el;
-      eloc[el] = make_int4(locA[th[e].x], locA[th[e].y], locB[e], 0);
+      eloc[el] = make_int4(locA[th[e].x] * Pn, locA[th[e].y] * Pn, locB[e] * Pm, 0);
     }
     floc.resize(2 * (size_t)nf);
     for (int fl = 0; fl < nf; ++fl) {
       const int f = fa + fl;
-      floc[2 * fl] = make_int4(locB[fe[f].x], locB[fe[f].y], locB[fe[f].z], S > 0 ? locA[fv[f].x] : 0);
-      floc[2 * fl + 1] = make_int4(S > 0 ? locA[fv[f].y] : 0, S > 0 ? locA[fv[f].z] : 0, 0, 0);
+      floc[2 * fl] = make_int4(locB[fe[f].x] * Pm, locB[fe[f].y] * Pm, locB[fe[f].z] * Pm, S > 0 ? locA[fv[f].x] * Pn : 0);
+      floc[2 * fl + 1] = make_int4(S > 0 ? locA[fv[f].y] * Pn : 0, S > 0 ? locA[fv[f].z] * Pn : 0, 0, 0);
     }
     head[kh_o_eloc] = blob_put(T.tab, base, eloc.data(), ne * sizeof(int4));
     head[kh_o_einv] = blob_put(T.tab, base, inv_theta.data() + ea, ne * (size_t)rb);
@@ -359,7 +371,7 @@ bool build_pipe_h(PipeTables& T, int n, int fpp, int nF, const std::vector<int>&
     const int end = head[kh_o_hnew] + (pipe::si_lane_groups(Tsi) ? (ne * rb + 15) / 16 * 16 : 0);
     if (round128(end) > max_stage) return false;  // the stage would not fit: stop early
     std::memcpy(T.tab.data() + base, head, sizeof(head));
-    T.desc.push_back(make_int4(kSrcTab, (int)(base / 16), 0, B));
+    T.desc.push_back(make_int4(kSrcTabH, (int)(base / 16), 0, B));
     add_runs(T.desc, kSrcEr, er_runs, head[kh_o_er], Pn * rb);
     add_runs(T.desc, kSrcEt, et_runs, head[kh_o_et], Pm * rb);
     if (ne > 0) T.desc.push_back(make_int4(kSrcHt, ea, head[kh_o_ht], ne * Pn * rb));
@@ -384,7 +396,7 @@ template <typename real>
 bool build_pipe_e(PipeTables& T, int n, const std::vector<int>& vptr, const std::vector<int>& vlist,
                   const std::vector<int>& eptr, const std::vector<int2>& lr, int SW, const std::vector<int>& ps_edge,
                   const std::vector<int>& ps_face, const std::vector<real>& ps_coef, const std::vector<real>& ps_wc,
-                  const std::vector<real>& inv_phi, const std::vector<real>& tn, bool plasma, int Pn, int Pm,
+                  const std::vector<real>& inv_phi, const std::vector<real>& tn, bool plasma, bool local, int Pn, int Pm,
                   const std::vector<char>& v_src, const std::vector<char>& e_src, std::vector<int>& locA,
                   std::vector<int>& locB, int max_stage, int min_gap) {
   using namespace pipe;
@@ -393,7 +405,7 @@ bool build_pipe_e(PipeTables& T, int n, const std::vector<int>& vptr, const std:
   std::vector<std::pair<int, int>> h_runs, f_runs, v_runs;
   std::vector<std::pair<int, int>> own;  // (vertex, slot)
   std::vector<int> vid, vh, vj;
-  std::vector<real> vcoef, vwc;
+  std::vector<real> vcoef, vwc, etan;
   std::vector<int4> eloc;
   vloc.assign(vlist.size(), 0);
   for (int q = 0; q < n; ++q) {
@@ -437,24 +449,31 @@ bool build_pipe_e(PipeTables& T, int n, const std::vector<int>& vptr, const std:
     vh.assign((size_t)nv * SW, 0);
     vj.assign((size_t)nv * SW, 0);
     vcoef.assign((size_t)nv * SW, real(0));
-    vwc.assign(plasma ? (size_t)nv * SW * 4 : 0, real(0));
+    // face frames: one weight per slot and four tangent components per edge are used (else 4, 8)
+    const size_t ws = local ? SW : 4 * SW, ts = local ? 4 : 8;
+    vwc.assign(plasma ? nv * ws : 0, real(0));
     for (int vl = 0; vl < nv; ++vl) {
       const int sl = own[vl].second;
       vid[vl] = own[vl].first;
       for (int k = 0; k < SW; ++k) {
         const size_t i = (size_t)sl * SW + k, o = (size_t)vl * SW + k;
-        vh[o] = locA[ps_edge[i]];
+        vh[o] = locA[ps_edge[i]] * Pn;
         vcoef[o] = ps_coef[i];
         if (plasma) {
-          vj[o] = locB[ps_face[i]];
-          for (int c = 0; c < 4; ++c) vwc[o * 4 + c] = ps_wc[i * 4 + c];
+          vj[o] = locB[ps_face[i]] * 3 * Pm;
+          if (!local)
+            for (int c = 0; c < 4; ++c) vwc[o * 4 + c] = ps_wc[i * 4 + c];
         }
       }
+      if (plasma && local) std::copy_n(ps_wc.begin() + (size_t)sl * SW * 4, SW, vwc.begin() + (size_t)vl * SW);
     }
+    etan.assign(plasma ? ne * ts : 0, real(0));
+    for (int el = 0; plasma && el < ne; ++el)
+      std::copy_n(tn.begin() + 8 * (size_t)(ea + el), ts, etan.begin() + el * ts);
     eloc.resize(ne);
     for (int el = 0; el < ne; ++el) {
       const int e = ea + el;
-      eloc[el] = make_int4(locA[e], locB[lr[e].x], locB[lr[e].y], 0);
+      eloc[el] = make_int4(locA[e] * Pn, locB[lr[e].x] * Pm, locB[lr[e].y] * Pm, 0);
     }
     head[ke_o_vid] = blob_put(T.tab, base, vid.data(), nv * sizeof(int));
     head[ke_o_vh] = blob_put(T.tab, base, vh.data(), vh.size() * sizeof(int));
@@ -463,7 +482,7 @@ bool build_pipe_e(PipeTables& T, int n, const std::vector<int>& vptr, const std:
     head[ke_o_vwc] = plasma ? blob_put(T.tab, base, vwc.data(), vwc.size() * (size_t)rb) : head[ke_o_vcoef];
     head[ke_o_eloc] = blob_put(T.tab, base, eloc.data(), ne * sizeof(int4));
     head[ke_o_einv] = blob_put(T.tab, base, inv_phi.data() + ea, ne * (size_t)rb);
-    head[ke_o_etan] = plasma ? blob_put(T.tab, base, tn.data() + 8 * (size_t)ea, 8 * (size_t)ne * rb) : head[ke_o_einv];
+    head[ke_o_etan] = plasma ? blob_put(T.tab, base, etan.data(), etan.size() * (size_t)rb) : head[ke_o_einv];
     const int B = (int)(T.tab.size() - base);
     head[ke_nv] = nv;
     head[ke_ea] = ea;
@@ -479,7 +498,7 @@ bool build_pipe_e(PipeTables& T, int n, const std::vector<int>& vptr, const std:
     const int end = head[ke_o_end];
     if (round128(end) > max_stage) return false;  // the stage would not fit: stop early
     std::memcpy(T.tab.data() + base, head, sizeof(head));
-    T.desc.push_back(make_int4(kSrcTab, (int)(base / 16), 0, B));
+    T.desc.push_back(make_int4(kSrcTabE, (int)(base / 16), 0, B));
     add_runs(T.desc, kSrcHt, h_runs, head[ke_o_ht], Pn * rb);
     add_runs(T.desc, kSrcHr, f_runs, head[ke_o_hr], Pm * rb);
     if (plasma) add_runs(T.desc, kSrcJsum, f_runs, head[ke_o_J], 3 * Pm * rb);
@@ -625,7 +644,7 @@ bool build_pipe_f(PipeTables& T, int n, const std::vector<int>& vptr, const std:
     const int end = head[kf_o_end];
     if (round128(end) > max_stage) return false;  // the stage would not fit: stop early
     std::memcpy(T.tab.data() + base, head, sizeof(head));
-    T.desc.push_back(make_int4(kSrcTab, (int)(base / 16), 0, B));
+    T.desc.push_back(make_int4(kSrcTabE, (int)(base / 16), 0, B));
     add_runs(T.desc, kSrcEr, v_runs, head[kf_o_er], Pn * rb);
     add_runs(T.desc, kSrcEt, t_runs, head[kf_o_et], Pm * rb);
     add_runs(T.desc, kSrcHt, h_runs, head[kf_o_ht], Pn * rb);
@@ -941,8 +960,8 @@ int build_plan(ifdtd_plan* P, const ifdtd_mesh_desc* M, const ifdtd_grid_desc* G
     auto a16 = [](long b) { return (b + 15) / 16 * 16; };
     auto bytes = [&](int h, int fcount, int v, int e) {
       long blob = 16L * ((pipe::ke_head_ints * 4 + 15) / 16) + a16(4L * v) + a16(4L * v * SW) * (with_plasma ? 2 : 1) + a16((long)rb * v * SW) +
-                  (with_plasma ? a16(4L * rb * v * SW) : 0) + a16(16L * e) + a16((long)rb * e) +
-                  (with_plasma ? a16(8L * rb * e) : 0);
+                  (with_plasma ? a16((local ? 1L : 4L) * rb * v * SW) : 0) + a16(16L * e) + a16((long)rb * e) +
+                  (with_plasma ? a16((local ? 4L : 8L) * rb * e) : 0);
       long rows = (long)rb * ((long)h * Pn + (long)fcount * Pm * (with_plasma ? 4 : 1) + (long)v * Pn + (long)e * Pm);
       return (blob + rows + 127) / 128 * 128;
     };
@@ -1119,7 +1138,8 @@ int build_plan(ifdtd_plan* P, const ifdtd_mesh_desc* M, const ifdtd_grid_desc* G
         const bool ok = build_pipe_f<real>(t, o.n, o.vptr, o.vlist, o.eptr, patch_of_edge, th, lr, fe, SW, sl.edge,
                                            sl.coef, inv_theta, inv_phi, fw, Pn, Pm, v_src, e_src, locV, locE, locH,
                                            locF, f_budget / 2);
-        if (!ok || 2 * t.stage_bytes > f_budget || !descriptors_valid(t, (int)sizeof(real), Pn, Pm, 0, nV, nE, nF, 0))
+        if (!ok || 2 * t.stage_bytes > f_budget ||
+            !finish_descriptors(t, pipe::kSrcTabE, {(int)sizeof(real), Pn, Pm, 0, nV, nE, nF, 0}))
           continue;
         fpp_e = c;
         oe = std::move(o);
@@ -1454,7 +1474,7 @@ int build_plan(ifdtd_plan* P, const ifdtd_mesh_desc* M, const ifdtd_grid_desc* G
       if (!build_slots(o.vlist, sl)) break;
       PipeTables t;
       const bool ok = build_pipe_e<real>(t, o.n, o.vptr, o.vlist, o.eptr, lr, SW, sl.edge, sl.face, sl.coef, sl.wc,
-                                         inv_phi, tn, plasma, Pn, Pm, v_src, e_src, locA, locB,
+                                         inv_phi, tn, plasma, local, Pn, Pm, v_src, e_src, locA, locB,
                                          stage_budget / stages_wanted, e_copy_gap);
       if (ok && stages_wanted * t.stage_bytes <= stage_budget) {
         P->pipe_e_ok = true;
@@ -1465,9 +1485,11 @@ int build_plan(ifdtd_plan* P, const ifdtd_mesh_desc* M, const ifdtd_grid_desc* G
         break;
       }
     }
-    if (P->pipe_h_ok && !descriptors_valid(th_tab, (int)sizeof(real), Pn, Pm, X->si_terms, nV, nE, nF, S))
+    if (P->pipe_h_ok &&
+        !finish_descriptors(th_tab, pipe::kSrcTabH, {(int)sizeof(real), Pn, Pm, X->si_terms, nV, nE, nF, S}))
       P->pipe_h_ok = false;
-    if (P->pipe_e_ok && !descriptors_valid(te_tab, (int)sizeof(real), Pn, Pm, 0, nV, nE, nF, plasma ? 1 : 0))
+    if (P->pipe_e_ok &&
+        !finish_descriptors(te_tab, pipe::kSrcTabE, {(int)sizeof(real), Pn, Pm, 0, nV, nE, nF, plasma ? 1 : 0}))
       P->pipe_e_ok = false;
     P->kh_stage = th_tab.stage_bytes;
     P->ke_stage = te_tab.stage_bytes;
@@ -1624,6 +1646,7 @@ int build_plan(ifdtd_plan* P, const ifdtd_mesh_desc* M, const ifdtd_grid_desc* G
     rb.et = (real*)P->fb[1];
     rb.hr = (real*)P->fb[2];
     rb.ht = (real*)P->fb[3];
+    pipe::set_sources(rb);
     cudaError_t e = A.alloc(sizeof(Rec<real>), &P->d_rec_b);
     if (e != cudaSuccess) return fail(IFDTD_ERR_CUDA, "allocation of the second launch record failed");
     CUDA_TRY(cudaMemcpy(P->d_rec_b, &rb, sizeof(rb), cudaMemcpyHostToDevice));
@@ -1647,6 +1670,7 @@ int bind_state(ifdtd_plan* P, const ifdtd_state* st, cudaStream_t stream) {
   R->ht = (real*)st->ht;
   R->si_mem = (real*)st->si_memory;
   for (int s = 0; s < kMaxSpecies; ++s) R->J[s] = (real*)st->plasma_current[s];
+  pipe::set_sources(*R);
   // pageable source: the runtime stages it before returning, so h_rec may change afterwards
   CUDA_TRY(cudaMemcpyAsync(P->d_rec, P->h_rec.data(), sizeof(Rec<real>), cudaMemcpyHostToDevice, stream));
   P->last_state = *st;
@@ -2344,6 +2368,7 @@ int run_batch(ifdtd_batch* B, const ifdtd_state* states, const double* currents,
       R->ht = (real*)s.ht;
       R->si_mem = (real*)s.si_memory;
       for (int k = 0; k < kMaxSpecies; ++k) R->J[k] = (real*)s.plasma_current[k];
+      pipe::set_sources(*R);
     }
     // pageable source: the runtime stages it before returning
     CUDA_TRY(cudaMemcpyAsync(B->d_recs, B->h_recs.data(), B->h_recs.size(), cudaMemcpyHostToDevice, stream));
@@ -2357,6 +2382,7 @@ int run_batch(ifdtd_batch* B, const ifdtd_state* states, const double* currents,
         R->et = (real*)P->fb[1];
         R->hr = (real*)P->fb[2];
         R->ht = (real*)P->fb[3];
+        pipe::set_sources(*R);
       }
       CUDA_TRY(cudaMemcpyAsync(B->d_recs_b, B->h_recs_b.data(), B->h_recs_b.size(), cudaMemcpyHostToDevice, stream));
     }
@@ -3053,6 +3079,7 @@ int step_static(ifdtd_plan* P, const ifdtd_state* st, const double* currents, in
   Rec<real> rec;
   std::memcpy(&rec, P->h_rec.data(), sizeof(rec));
   rec.Jtot = P->S > 1 ? static_cast<real*>(A.scratch) : nullptr;
+  pipe::set_sources(rec);
   rec.cur = currents ? currents : static_cast<const double*>(A.zero_current);
   std::memcpy(bytes, &rec, sizeof(rec));
   // the summed current is fully rewritten each step; clearing it keeps a call

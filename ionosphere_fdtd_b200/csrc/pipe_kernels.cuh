@@ -38,8 +38,30 @@ constexpr int kWideRegs = 96;
 constexpr int kWideMaxThreads = 640;
 constexpr uint64_t kWaitNs = 500ull * 1000 * 1000;  // bound of one wait (0.5 s)
 
-// Descriptor sources (int4 {src, first row, stage byte offset, bytes}).
-enum Src : int { kSrcEr = 0, kSrcEt = 1, kSrcHt = 2, kSrcHr = 3, kSrcJsum = 4, kSrcTab = 5, kSrcSi = 6, kSrcJ0 = 8 };
+// Descriptor sources (int4 {src, offset in the source in 16-byte units, stage
+// byte offset, bytes}): an index into the record's base pointers, so a copy's
+// address is one load and one multiply-add, the same for every lane.  A switch over
+// the arrays, which the lanes took one after the other, held back the copies: E
+// phase 123 -> 111 us at s7 / 40 cells, 837 -> 776 at s8 / 80, H phase without
+// plasma 86 -> 76 at s7 / 40.
+enum Src : int {
+  kSrcEr = 0, kSrcEt = 1, kSrcHt = 2, kSrcHr = 3, kSrcJsum = 4, kSrcTabH = 5, kSrcSi = 6, kSrcTabE = 7, kSrcJ0 = 8
+};
+static_assert(kSrcJ0 + kMaxSpecies <= kSources, "source table too small");
+
+// The base pointers of a record whose state or table pointers changed (host).
+template <typename real>
+void set_sources(Rec<real>& R) {
+  R.src[kSrcEr] = R.er;
+  R.src[kSrcEt] = R.et;
+  R.src[kSrcHt] = R.ht;
+  R.src[kSrcHr] = R.hr;
+  R.src[kSrcJsum] = R.n_species > 1 ? R.Jtot : R.J[0];
+  R.src[kSrcTabH] = R.tab_h;
+  R.src[kSrcSi] = R.si_mem;
+  R.src[kSrcTabE] = R.tab_e;
+  for (int s = 0; s < kMaxSpecies; ++s) R.src[kSrcJ0 + s] = R.J[s];
+}
 
 // H-phase blob header (ints; offsets are bytes from the stage start).
 enum KhHead : int {
@@ -146,18 +168,8 @@ struct Ring {
 };
 
 template <typename real>
-__device__ __forceinline__ const void* desc_source(const Rec<real>& R, const unsigned char* tab, int src, int row) {
-  const size_t r = (size_t)row;
-  switch (src) {
-    case kSrcEr: return R.er + r * R.Pn;
-    case kSrcEt: return R.et + r * R.Pm;
-    case kSrcHt: return R.ht + r * R.Pn;
-    case kSrcHr: return R.hr + r * R.Pm;
-    case kSrcJsum: return jsum(R) + r * 3 * R.Pm;
-    case kSrcTab: return tab + r * 16;
-    case kSrcSi: return R.si_mem + r * R.si_terms;
-    default: return R.J[(src - kSrcJ0) & (kMaxSpecies - 1)] + r * 3 * R.Pm;
-  }
+__device__ __forceinline__ const unsigned char* desc_source(const Rec<real>& R, int src, int units) {
+  return static_cast<const unsigned char*>(R.src[src]) + (size_t)(uint32_t)units * 16;
 }
 
 // Producer warp w of W: fills stage i % n_stages with its share (descriptors
@@ -171,7 +183,7 @@ __device__ __forceinline__ const void* desc_source(const Rec<real>& R, const uns
 // completion by one cp.async arrival per producer lane.
 template <int COPY, typename real>
 __device__ void produce(const Rec<real>& R, const Ring& G, int p0, int p1, int n_patches, const int* dptr,
-                        const int4* desc, const unsigned char* tab, int w, int W) {
+                        const int4* desc, int w, int W) {
   const int lane = threadIdx.x & 31;
   int win = p0;
   int dpw = __ldg(dptr + min(win + lane, n_patches));
@@ -212,7 +224,7 @@ __device__ void produce(const Rec<real>& R, const Ring& G, int p0, int p1, int n
 #pragma unroll
       for (int k = 0; k < kDescPerLane; ++k)
         if (w + W * (lane + 32 * k) < ncur)
-          bulk_load(st + cur[k].z, desc_source(R, tab, cur[k].x, cur[k].y), (uint32_t)cur[k].w, G.full + s);
+          bulk_load(st + cur[k].z, desc_source(R, cur[k].x, cur[k].y), (uint32_t)cur[k].w, G.full + s);
     } else {
 #pragma unroll
       for (int k = 0; k < kDescPerLane; ++k) {
@@ -220,10 +232,10 @@ __device__ void produce(const Rec<real>& R, const Ring& G, int p0, int p1, int n
         const int nk = max(0, min(32, (ncur - w + W - 1) / W - 32 * k));
         for (int j = 0; j < nk; ++j) {
           const int src = __shfl_sync(0xFFFFFFFFu, cur[k].x, j);
-          const int row = __shfl_sync(0xFFFFFFFFu, cur[k].y, j);
+          const int units = __shfl_sync(0xFFFFFFFFu, cur[k].y, j);
           const int dst = __shfl_sync(0xFFFFFFFFu, cur[k].z, j);
           const int bytes = __shfl_sync(0xFFFFFFFFu, cur[k].w, j);
-          const unsigned char* sp = static_cast<const unsigned char*>(desc_source(R, tab, src, row));
+          const unsigned char* sp = desc_source(R, src, units);
           for (int c = lane * 16; c < bytes; c += 32 * 16) cp16_async(st + dst + c, sp + c);
         }
       }
@@ -285,11 +297,55 @@ __device__ __forceinline__ LaneMap lane_map(int ct, int nct, int c, int layout) 
   return m;
 }
 
-template <typename real, bool PLASMA>
-__device__ __forceinline__ void kh_consume(const Rec<real>& R, const Layers<real>& Ls, unsigned char* st, int ct,
-                                           int nct, uint64_t* group, uint32_t ph, const Ring& G, int layout) {
+// A patch gives a thread about six runs, so what it does once per patch counts:
+// the lane maps (integer divisions) and the layer factors of its radial quads stay
+// in registers over all patches, a patch's header is read as 16-byte vectors, and
+// its tables hold element offsets rather than row numbers.  Done per patch and run,
+// these were 9 of 60 million warp instructions of the E phase at s7 / 40 cells and 7
+// of 57 of the H phase (E 131 -> 123 us, H 129 -> 125; s8 / 80 E 895 -> 837, H 975 ->
+// 940).
+template <int N>
+__device__ __forceinline__ void load_head(const unsigned char* st, int (&h)[N]) {
+  static_assert(N % 4 == 0, "whole vectors");
+#pragma unroll
+  for (int i = 0; i < N; i += 4) {
+    const int4 x = *reinterpret_cast<const int4*>(st + 4 * i);
+    h[i] = x.x;
+    h[i + 1] = x.y;
+    h[i + 2] = x.z;
+    h[i + 3] = x.w;
+  }
+}
+
+// A thread's rows in the H consumers: node quads of the edges, midpoint quads of
+// the faces, and their layer factors.
+template <typename real>
+struct HLanes {
+  LaneMap edge, face;
+  int edge0, face0;  // first row
+  HEdgeLayer<real> ey;
+  Run<real> fc;
+};
+template <typename real>
+__device__ __forceinline__ HLanes<real> h_lanes(const Rec<real>& R, const Layers<real>& Ls, int ct, int nct, int layout) {
   constexpr int N = Lanes<real>::N;
-  const int* hd = reinterpret_cast<const int*>(st);
+  HLanes<real> m{};
+  m.edge = lane_map(ct, nct, R.Pn / N, layout);
+  m.face = lane_map(ct, nct, R.Pm / N, layout);
+  m.edge0 = ct / m.edge.G;
+  m.face0 = ct / m.face.G;
+  if (m.edge.on) m.ey = h_edge_layer(R, Ls, m.edge.q * N);
+  if (m.face.on) m.fc = ld16(Ls.hC + m.face.q * N);
+  return m;
+}
+
+template <typename real, bool PLASMA>
+__device__ __forceinline__ void kh_consume(const Rec<real>& R, const Layers<real>& Ls, const HLanes<real>& lanes,
+                                           unsigned char* st, int ct, int nct, uint64_t* group, uint32_t ph,
+                                           const Ring& G) {
+  constexpr int N = Lanes<real>::N;
+  int hd[kh_head_ints];
+  load_head(st, hd);
   const int ea = hd[kh_ea], ne = hd[kh_ne], fa = hd[kh_fa], nf = hd[kh_nf];
   const real* s_er = reinterpret_cast<const real*>(st + hd[kh_o_er]);
   const real* s_et = reinterpret_cast<const real*>(st + hd[kh_o_et]);
@@ -306,15 +362,15 @@ __device__ __forceinline__ void kh_consume(const Rec<real>& R, const Layers<real
   real* s_hnew = reinterpret_cast<real*>(st + hd[kh_o_hnew]);
   const int T = R.si_terms;
   const bool si_pass = si_lane_groups(T);
-  const int Pn = R.Pn, Pm = R.Pm, cn = Pn / N, cm = Pm / N;
+  const int Pn = R.Pn, Pm = R.Pm;
   if (si_pass) {
     // each owned edge's surface-impedance ADE on T/4 lanes (four poles each):
     // partial history sums gathered in pole order, the node-0 Ht into the
     // stage's scratch, then all compute warps meet on the slot's group barrier
-    const int Q = T / 4, lane = threadIdx.x & 31, n_it = ne * Q;
+    const int Q = T / 4, lane = threadIdx.x & 31, n_it = ne * Q, log_q = 31 - __clz(Q);
     for (int base = ct - lane; base < n_it; base += nct) {
       const int it = min(base + lane, n_it - 1);
-      const int el = it / Q, qd = it - el * Q;
+      const int el = it >> log_q, qd = it - (el << log_q);
       const int e = ea + el;
       const int4 loc = eloc[el];
       const real* mem = s_si + el * T;
@@ -323,8 +379,8 @@ __device__ __forceinline__ void kh_consume(const Rec<real>& R, const Layers<real
       real hist = __shfl_sync(0xFFFFFFFFu, part, first);
       for (int q = 1; q < Q; ++q) hist = add_rn(hist, __shfl_sync(0xFFFFFFFFu, part, first + q));
       const real h_old = s_ht[el * Pn];
-      const real g0 = (s_er[loc.y * Pn] - s_er[loc.x * Pn]) * einv[el] * Ls.invr[0];
-      const real e1 = R.si_metric * s_et[loc.z * Pm];
+      const real g0 = (s_er[loc.y] - s_er[loc.x]) * einv[el] * Ls.invr[0];
+      const real e1 = R.si_metric * s_et[loc.z];
       const real h_new = si_boundary(R, h_old, g0, e1, esis[el], hist);
       if (base + lane < n_it) {
         si_update_quad(mem + 4 * qd, R.si_mem + (size_t)e * T + 4 * qd, Ls, 4 * qd, h_new + h_old);
@@ -335,50 +391,70 @@ __device__ __forceinline__ void kh_consume(const Rec<real>& R, const Layers<real
     if ((threadIdx.x & 31) == 0) mbar_arrive(group);
     if (!__all_sync(0xFFFFFFFFu, wait_phase(group, ph, G.abort_flag, G.status))) return;
   }
-  // edge runs (nodes) and face runs (midpoints), each thread on a fixed
-  // radial quad (layer factors loaded once per patch; see ke_consume)
-  {
-    const LaneMap lm = lane_map(ct, nct, cn, layout);
-    if (lm.on) {
-      const int k0 = lm.q * N;
-      const HEdgeLayer<real> y = h_edge_layer(R, Ls, k0);
-      for (int el = ct / lm.G; el < ne; el += lm.per) {
-        const int e = ea + el;
-        const int4 loc = eloc[el];
-        h_edge_run(R, Ls, y, e, k0, s_er + loc.y * Pn, s_er + loc.x * Pn, s_et + loc.z * Pm, s_ht + el * Pn,
-                   R.ht + (size_t)e * Pn, einv[el], s_si + el * T, R.si_mem + (size_t)e * T, esis + el,
-                   si_pass ? s_hnew + el : nullptr);
-      }
+  // edge runs (nodes) and face runs (midpoints), each thread on its radial quads
+  if (lanes.edge.on) {
+    const int k0 = lanes.edge.q * N;
+    for (int el = lanes.edge0; el < ne; el += lanes.edge.per) {
+      const int e = ea + el;
+      const int4 loc = eloc[el];
+      h_edge_run(R, Ls, lanes.ey, e, k0, s_er + loc.y, s_er + loc.x, s_et + loc.z, s_ht + el * Pn,
+                 R.ht + (size_t)e * Pn, einv[el], s_si + el * T, R.si_mem + (size_t)e * T, esis + el,
+                 si_pass ? s_hnew + el : nullptr);
     }
   }
-  {
-    const LaneMap lm = lane_map(ct, nct, cm, layout);
-    if (lm.on) {
-      const int j0 = lm.q * N;
-      const Run<real> fc = ld16(Ls.hC + j0);
-      for (int fl = ct / lm.G; fl < nf; fl += lm.per) {
-        const int f = fa + fl;
-        const int4 l0 = floc[2 * fl];
-        const int4 l1 = floc[2 * fl + 1];
-        h_face_run<real, PLASMA>(R, Ls, fc, f, j0, s_et + l0.x * Pm, s_et + l0.y * Pm, s_et + l0.z * Pm,
-                                 s_hr + fl * Pm, R.hr + (size_t)f * Pm, s_er + l0.w * Pn, s_er + l1.x * Pn,
-                                 s_er + l1.y * Pn, s_J + fl * 3 * Pm, nf * 3 * Pm,
-                                 R.n_species > 1 ? R.Jtot + (size_t)f * 3 * Pm : nullptr, fw + 4 * fl, fpl + 12 * fl);
-      }
+  if (lanes.face.on) {
+    const int j0 = lanes.face.q * N;
+    for (int fl = lanes.face0; fl < nf; fl += lanes.face.per) {
+      const int f = fa + fl;
+      const int4 l0 = floc[2 * fl];
+      const int4 l1 = floc[2 * fl + 1];
+      h_face_run<real, PLASMA>(R, Ls, lanes.fc, f, j0, s_et + l0.x, s_et + l0.y, s_et + l0.z, s_hr + fl * Pm,
+                               R.hr + (size_t)f * Pm, s_er + l0.w, s_er + l1.x, s_er + l1.y, s_J + fl * 3 * Pm,
+                               nf * 3 * Pm, R.n_species > 1 ? R.Jtot + (size_t)f * 3 * Pm : nullptr, fw + 4 * fl,
+                               fpl + 12 * fl);
     }
   }
 }
 
-// E phase of one patch from its stage (same arithmetic as ke_kernel).  Each
-// loop gives every thread a fixed radial quad: thread ct takes quad ct % c of
-// entities ct / c, ct / c + per, ... (c quads per row, per = nct / c entities
-// per sweep; threads from per * c on sit the loop out), so the per-layer
-// factors of its quad load once per patch instead of once per run.
-template <typename real, bool PLASMA, int MAXDEG>
-__device__ __forceinline__ void ke_consume(const Rec<real>& R, const Layers<real>& Ls, unsigned char* st, int ct,
-                                           int nct, real current, int layout, unsigned pattern) {
+// E phase of one patch from its stage (same arithmetic as ke_kernel).  Every
+// thread has a fixed radial quad in each loop: thread ct takes quad ct % c of
+// entities ct / c, ct / c + per, ... (c quads per row, per = nct / c entities per
+// sweep; threads from per * c on sit the loop out).  The vertex layer factors stay
+// in registers in the float kernels of vertex degree 6; elsewhere (float64,
+// 12-slot tables) holding them would push the kernel past its register budget
+// into local memory, so they are re-read per run.
+template <typename real, int MAXDEG>
+constexpr bool kHoistVertex = sizeof(real) == 4 && MAXDEG == 6;
+template <typename real>
+struct ELanes {
+  LaneMap vertex, edge;
+  int vertex0, edge0;  // first row
+  VertexLayer<real> vy;
+  EdgeLayer<real> ey;
+  unsigned pattern;  // lanes of this warp that hold a vertex quad
+};
+template <typename real, int MAXDEG>
+__device__ __forceinline__ ELanes<real> e_lanes(const Rec<real>& R, const Layers<real>& Ls, int ct, int nct, int layout) {
   constexpr int N = Lanes<real>::N;
-  const int* hd = reinterpret_cast<const int*>(st);
+  ELanes<real> m{};
+  m.vertex = lane_map(ct, nct, R.Pn / N, layout);
+  m.edge = lane_map(ct, nct, R.Pm / N, layout);
+  m.vertex0 = ct / m.vertex.G;
+  m.edge0 = ct / m.edge.G;
+  if (!R.coef_full) {
+    if (kHoistVertex<real, MAXDEG> && m.vertex.on) m.vy = vertex_layer(R, Ls, 0, m.vertex.q * N);
+    if (m.edge.on) m.ey = edge_layer(R, Ls, 0, m.edge.q * N);
+  }
+  m.pattern = __ballot_sync(0xFFFFFFFFu, m.vertex.on);
+  return m;
+}
+
+template <typename real, bool PLASMA, int MAXDEG>
+__device__ __forceinline__ void ke_consume(const Rec<real>& R, const Layers<real>& Ls, const ELanes<real>& lanes,
+                                           unsigned char* st, int ct, real current) {
+  constexpr int N = Lanes<real>::N;
+  int hd[ke_head_ints];
+  load_head(st, hd);
   const int nv = hd[ke_nv], ea = hd[ke_ea], ne = hd[ke_ne], src = hd[ke_src];
   const real* s_ht = reinterpret_cast<const real*>(st + hd[ke_o_ht]);
   const real* s_hr = reinterpret_cast<const real*>(st + hd[ke_o_hr]);
@@ -393,106 +469,81 @@ __device__ __forceinline__ void ke_consume(const Rec<real>& R, const Layers<real
   const int4* eloc = reinterpret_cast<const int4*>(st + hd[ke_o_eloc]);
   const real* einv = reinterpret_cast<const real*>(st + hd[ke_o_einv]);
   const real* etan = reinterpret_cast<const real*>(st + hd[ke_o_etan]);
-  const int Pn = R.Pn, Pm = R.Pm, SW = R.slot_width, cn = Pn / N, cm = Pm / N;
+  const int Pn = R.Pn, Pm = R.Pm;
+  constexpr int SW = (MAXDEG + 3) / 4 * 4;
   const bool full = R.coef_full != 0;
   const bool local = PLASMA && R.plasma_local != 0;
+  const int w_stride = local ? SW : 4 * SW, t_stride = local ? 4 : 8;  // reals per vertex, per edge
   auto slot_rows = [&](int vl, const real** hrows, const real** jrows) {
 #pragma unroll
     for (int q = 0; q < MAXDEG; q += 4) {
       const int4 h4 = *reinterpret_cast<const int4*>(vh + vl * SW + q);
-      hrows[q] = s_ht + h4.x * Pn;
-      hrows[q + 1] = s_ht + h4.y * Pn;
-      if (q + 2 < MAXDEG) hrows[q + 2] = s_ht + h4.z * Pn;
-      if (q + 3 < MAXDEG) hrows[q + 3] = s_ht + h4.w * Pn;
+      hrows[q] = s_ht + h4.x;
+      hrows[q + 1] = s_ht + h4.y;
+      if (q + 2 < MAXDEG) hrows[q + 2] = s_ht + h4.z;
+      if (q + 3 < MAXDEG) hrows[q + 3] = s_ht + h4.w;
       if (PLASMA) {
         const int4 j4 = *reinterpret_cast<const int4*>(vj + vl * SW + q);
-        jrows[q] = s_J + j4.x * 3 * Pm;
-        jrows[q + 1] = s_J + j4.y * 3 * Pm;
-        if (q + 2 < MAXDEG) jrows[q + 2] = s_J + j4.z * 3 * Pm;
-        if (q + 3 < MAXDEG) jrows[q + 3] = s_J + j4.w * 3 * Pm;
+        jrows[q] = s_J + j4.x;
+        jrows[q + 1] = s_J + j4.y;
+        if (q + 2 < MAXDEG) jrows[q + 2] = s_J + j4.z;
+        if (q + 3 < MAXDEG) jrows[q + 3] = s_J + j4.w;
       } else {
         for (int i = 0; i < 4 && q + i < MAXDEG; ++i) jrows[q + i] = nullptr;
       }
     }
   };
-  {
-    // vertex runs: thread ct holds node quad q of its vertices.  With plasma
-    // it computes the vertex's radial current on midpoint quad q itself
-    // (midpoints k0 .. k0+N-1) and takes the one below, k0-1, from lane - 1,
-    // which holds quad q-1 of the same vertex; a lane whose quad q-1 sits in
-    // the previous warp (lane 0) computes that value directly
-    const LaneMap lm = lane_map(ct, nct, cn, layout);
-    if (lm.on) {
-      const int q = lm.q, k0 = q * N, per = lm.per;
-      const int lane = threadIdx.x & 31, wbase = ct - lane;
-      // the vertex layer factors of this thread's quad: loaded once per patch
-      // in the float kernels of vertex degree 6 when they are altitude rows;
-      // elsewhere (float64, 12-slot tables) holding them would push the kernel
-      // past its register budget into local memory, so they are re-read per run
-      constexpr bool kHoist = sizeof(real) == 4 && MAXDEG == 6;
-      VertexLayer<real> fixed_v{};
-      if (kHoist && !full) fixed_v = vertex_layer(R, Ls, 0, k0);
-      for (int k = 0;; ++k) {
-        const int vl = ct / lm.G + k * per;
-        if (vl >= nv) break;
-        // lanes in this iteration: those of the pattern (a valid quad of a
-        // row slot) whose thread index is below the sweep's limit
-        const int cnt = min(per, nv - k * per) * lm.G - wbase;
-        const unsigned mask = pattern & (cnt >= 32 ? 0xFFFFFFFFu : ((1u << cnt) - 1u));
-        const int v = vid[vl];
-        const real* hrows[MAXDEG];
-        const real* jrows[MAXDEG];
-        slot_rows(vl, hrows, jrows);
-        real rav[N + 1];
-        if (PLASMA) {
-          const real* wcs = vwc + vl * SW * 4;
-          Run<real> own = zero_run<real>();
-          if (local) {
-            if (k0 < Pm) own = vertex_radial_current_local<real, MAXDEG>(jrows, wcs, k0);
-          } else if (k0 < Pm) {
-            own = vertex_radial_current<real, MAXDEG>(jrows, wcs, k0, Pm);
-          }
-          const real below = __shfl_up_sync(mask, own.x[N - 1], 1);
-          rav[0] = q == 0   ? real(0)
-                   : lane > 0 ? below
-                   : local    ? vertex_radial_current_local_at<real, MAXDEG>(jrows, wcs, k0 - 1)
-                              : vertex_radial_current_at<real, MAXDEG>(jrows, wcs, k0 - 1, Pm);
-#pragma unroll
-          for (int r = 0; r < N; ++r) rav[r + 1] = own.x[r];
+  // vertex runs: thread ct holds node quad q of its vertices.  With plasma it
+  // computes the vertex's radial current on midpoint quad q itself (midpoints
+  // k0 .. k0+N-1) and takes the one below, k0-1, from lane - 1, which holds quad
+  // q-1 of the same vertex; a lane whose quad q-1 sits in the previous warp (lane
+  // 0) computes that value directly
+  if (lanes.vertex.on) {
+    const int q = lanes.vertex.q, k0 = q * N, per = lanes.vertex.per;
+    const int lane = threadIdx.x & 31, wbase = ct - lane;
+    // lanes of a sweep: those of the pattern whose thread index is below its limit
+    int left = nv * lanes.vertex.G - wbase;
+    const int sweep = per * lanes.vertex.G;
+    for (int vl = lanes.vertex0; vl < nv; vl += per, left -= sweep) {
+      const unsigned mask = lanes.pattern & (left >= 32 ? 0xFFFFFFFFu : ((1u << left) - 1u));
+      const int v = vid[vl];
+      const real* hrows[MAXDEG];
+      const real* jrows[MAXDEG];
+      slot_rows(vl, hrows, jrows);
+      real rav[N + 1];
+      if (PLASMA) {
+        const real* wcs = vwc + vl * w_stride;
+        Run<real> own = zero_run<real>();
+        if (local) {
+          if (k0 < Pm) own = vertex_radial_current_local<real, MAXDEG>(jrows, wcs, k0);
+        } else if (k0 < Pm) {
+          own = vertex_radial_current<real, MAXDEG>(jrows, wcs, k0, Pm);
         }
-        e_vertex_run<real, PLASMA, MAXDEG>(R, kHoist && !full ? fixed_v : vertex_layer(R, Ls, v, k0), (src & 1) != 0, v, k0, hrows,
-                                           jrows, vcoef + vl * SW, PLASMA ? vwc + vl * SW * 4 : nullptr,
-                                           s_er + vl * Pn, R.er + (size_t)v * Pn, current, PLASMA ? rav : nullptr);
+        const real below = __shfl_up_sync(mask, own.x[N - 1], 1);
+        rav[0] = q == 0   ? real(0)
+                 : lane > 0 ? below
+                 : local    ? vertex_radial_current_local_at<real, MAXDEG>(jrows, wcs, k0 - 1)
+                            : vertex_radial_current_at<real, MAXDEG>(jrows, wcs, k0 - 1, Pm);
+#pragma unroll
+        for (int r = 0; r < N; ++r) rav[r + 1] = own.x[r];
       }
+      e_vertex_run<real, PLASMA, MAXDEG>(R, kHoistVertex<real, MAXDEG> && !full ? lanes.vy : vertex_layer(R, Ls, v, k0),
+                                         (src & 1) != 0, v, k0, hrows, jrows, vcoef + vl * SW,
+                                         PLASMA ? vwc + vl * w_stride : nullptr, s_er + vl * Pn,
+                                         R.er + (size_t)v * Pn, current, PLASMA ? rav : nullptr);
     }
   }
-  {
-    const LaneMap lm = lane_map(ct, nct, cm, layout);
-    if (lm.on) {
-      const int j0 = lm.q * N;
-      const EdgeLayer<real> fixed = edge_layer(R, Ls, ea, j0);
-      for (int el = ct / lm.G; el < ne; el += lm.per) {
-        const int e = ea + el;
-        const int4 loc = eloc[el];
-        e_edge_run<real, PLASMA>(R, full ? edge_layer(R, Ls, e, j0) : fixed, (src & 2) != 0, e, j0,
-                                 s_hr + loc.y * Pm, s_hr + loc.z * Pm, s_ht + loc.x * Pn,
-                                 PLASMA ? s_J + loc.y * 3 * Pm : nullptr, PLASMA ? s_J + loc.z * 3 * Pm : nullptr,
-                                 s_et + el * Pm, R.et + (size_t)e * Pm, current, einv[el],
-                                 PLASMA ? etan + el * 8 : nullptr);
-      }
+  if (lanes.edge.on) {
+    const int j0 = lanes.edge.q * N;
+    for (int el = lanes.edge0; el < ne; el += lanes.edge.per) {
+      const int e = ea + el;
+      const int4 loc = eloc[el];
+      e_edge_run<real, PLASMA>(R, full ? edge_layer(R, Ls, e, j0) : lanes.ey, (src & 2) != 0, e, j0, s_hr + loc.y,
+                               s_hr + loc.z, s_ht + loc.x, PLASMA ? s_J + loc.y * 3 : nullptr,
+                               PLASMA ? s_J + loc.z * 3 : nullptr, s_et + el * Pm, R.et + (size_t)e * Pm, current,
+                               einv[el], PLASMA ? etan + el * t_stride : nullptr);
     }
   }
-}
-
-// Bit l set when lane l of this thread's warp holds a valid quad (q < c) in
-// the vertex-run lane map: the shuffle mask of the lanes that take part in a
-// sweep, before the sweep's row limit is applied.
-__device__ __forceinline__ unsigned lane_pattern(int ct, int nct, int c, int layout) {
-  const int wbase = ct - (threadIdx.x & 31);
-  unsigned bits = 0;
-  for (int l = 0; l < 32; ++l)
-    if (lane_map(wbase + l, nct, c, layout).on) bits |= 1u << l;
-  return bits;
 }
 
 // Shared prologue: barriers, record and ring.  The per-layer rows are the
@@ -547,13 +598,14 @@ __global__ void __maxnreg__(kMaxRegs) kh_tma(const Rec<real>* __restrict__ recs,
   const int n = R.n_patches_h;
   const int p0 = (int)((long long)n * blockIdx.x / gridDim.x), p1 = (int)((long long)n * (blockIdx.x + 1) / gridDim.x);
   if (threadIdx.x < 32 * W) {
-    produce<COPY>(R, G, p0, p1, n, R.dptr_h, R.desc_h, R.tab_h, threadIdx.x / 32, W);
+    produce<COPY>(R, G, p0, p1, n, R.dptr_h, R.desc_h, threadIdx.x / 32, W);
   } else {
     const int ct = threadIdx.x - 32 * W, nct = blockDim.x - 32 * W;
     Layers<real> Ls;
     consumer_layers(R, dyn_smem, Ls, ct, nct);
+    const HLanes<real> lanes = h_lanes(R, Ls, ct, nct, layout);
     consume_ring(G, p0, p1, [&](unsigned char* st, int s, uint32_t ph) {
-      kh_consume<real, PLASMA>(R, Ls, st, ct, nct, group + s, ph, G, layout);
+      kh_consume<real, PLASMA>(R, Ls, lanes, st, ct, nct, group + s, ph, G);
     });
   }
 }
@@ -571,15 +623,15 @@ __global__ void __maxnreg__(REGS) ke_tma(const Rec<real>* __restrict__ recs, int
   const int n = R.n_patches_e;
   const int p0 = (int)((long long)n * blockIdx.x / gridDim.x), p1 = (int)((long long)n * (blockIdx.x + 1) / gridDim.x);
   if (threadIdx.x < 32 * W) {
-    produce<COPY>(R, G, p0, p1, n, R.dptr_e, R.desc_e, R.tab_e, threadIdx.x / 32, W);
+    produce<COPY>(R, G, p0, p1, n, R.dptr_e, R.desc_e, threadIdx.x / 32, W);
   } else {
     const int ct = threadIdx.x - 32 * W, nct = blockDim.x - 32 * W;
     Layers<real> Ls;
     consumer_layers(R, dyn_smem, Ls, ct, nct);
     const real current = (R.n_src_er + R.n_src_et) > 0 ? (real)R.cur[istep] : real(0);
-    const unsigned pattern = lane_pattern(ct, nct, R.Pn / Lanes<real>::N, layout);
+    const ELanes<real> lanes = e_lanes<real, MAXDEG>(R, Ls, ct, nct, layout);
     consume_ring(G, p0, p1, [&](unsigned char* st, int s, uint32_t ph) {
-      ke_consume<real, PLASMA, MAXDEG>(R, Ls, st, ct, nct, current, layout, pattern);
+      ke_consume<real, PLASMA, MAXDEG>(R, Ls, lanes, st, ct, current);
     });
   }
 }
@@ -628,13 +680,14 @@ __global__ void __maxnreg__(kMaxRegs) kh_tma_batch(const Rec<real>* __restrict__
     Ring G;
     ring_setup(R, recs + sg.x, dyn_smem, full, empty, &abort_flag, rg.x, rg.y, COPY == 0 ? W : 32 * W, W, G);
     if (threadIdx.x < 32 * W) {
-      produce<COPY>(R, G, sg.y, sg.z, R.n_patches_h, R.dptr_h, R.desc_h, R.tab_h, threadIdx.x / 32, W);
+      produce<COPY>(R, G, sg.y, sg.z, R.n_patches_h, R.dptr_h, R.desc_h, threadIdx.x / 32, W);
     } else {
       const int ct = threadIdx.x - 32 * W, nct = blockDim.x - 32 * W;
       Layers<real> Ls;
       consumer_layers(R, dyn_smem, Ls, ct, nct);
+      const HLanes<real> lanes = h_lanes(R, Ls, ct, nct, layout);
       consume_ring(G, sg.y, sg.z, [&](unsigned char* st, int s, uint32_t ph) {
-        kh_consume<real, PLASMA>(R, Ls, st, ct, nct, group + s, ph, G, layout);
+        kh_consume<real, PLASMA>(R, Ls, lanes, st, ct, nct, group + s, ph, G);
       });
     }
   }
@@ -661,15 +714,15 @@ __global__ void __maxnreg__(REGS) ke_tma_batch(const Rec<real>* __restrict__ rec
     Ring G;
     ring_setup(R, recs + sg.x, dyn_smem, full, empty, &abort_flag, rg.x, rg.y, COPY == 0 ? W : 32 * W, W, G);
     if (threadIdx.x < 32 * W) {
-      produce<COPY>(R, G, sg.y, sg.z, R.n_patches_e, R.dptr_e, R.desc_e, R.tab_e, threadIdx.x / 32, W);
+      produce<COPY>(R, G, sg.y, sg.z, R.n_patches_e, R.dptr_e, R.desc_e, threadIdx.x / 32, W);
     } else {
       const int ct = threadIdx.x - 32 * W, nct = blockDim.x - 32 * W;
       Layers<real> Ls;
       consumer_layers(R, dyn_smem, Ls, ct, nct);
       const real current = (R.n_src_er + R.n_src_et) > 0 ? (real)R.cur[istep] : real(0);
-      const unsigned pattern = lane_pattern(ct, nct, R.Pn / Lanes<real>::N, layout);
+      const ELanes<real> lanes = e_lanes<real, MAXDEG>(R, Ls, ct, nct, layout);
       consume_ring(G, sg.y, sg.z, [&](unsigned char* st, int s, uint32_t ph) {
-        ke_consume<real, PLASMA, MAXDEG>(R, Ls, st, ct, nct, current, layout, pattern);
+        ke_consume<real, PLASMA, MAXDEG>(R, Ls, lanes, st, ct, current);
       });
     }
   }

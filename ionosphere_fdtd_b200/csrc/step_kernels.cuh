@@ -38,6 +38,7 @@ namespace ifdtd {
 
 constexpr int kMaxSpecies = 4;
 constexpr int kMaxSources = 16;
+constexpr int kSources = 12;
 
 template <typename real>
 struct Rec {
@@ -56,6 +57,7 @@ struct Rec {
   real *er, *et, *hr, *ht, *si_mem;
   real* J[kMaxSpecies];  // (F, 3, Pm) per species
   real* Jtot;            // summed species current when n_species > 1
+  const void* src[kSources];  // base of each copy source (pipe::Src; set_sources)
   const double* cur;     // per-step source current (staging row)
   int* status;           // device status word (bit 0: a staging wait timed out)
   // ownership: H phase patches own faces [p*fpp_h, ...) and eptr_h edges;
