@@ -1089,21 +1089,33 @@ __global__ void sample_batch_kernel(const Rec<real>* __restrict__ recs, const Pr
 // max |x| of up to four arrays; results combined with an order-independent
 // atomic max on the bit pattern of non-negative doubles (NaN sorts above +Inf,
 // so a non-finite field reports NaN or Inf).  Row padding is zero and does not
-// change a maximum of absolute values.
+// change a maximum of absolute values.  Bound by the reads: 16-byte loads, four in
+// flight per thread.
 template <typename real>
 __global__ void max_abs_kernel(const real* __restrict__ a0, size_t n0, const real* __restrict__ a1, size_t n1,
                                const real* __restrict__ a2, size_t n2, const real* __restrict__ a3, size_t n3,
                                unsigned long long* __restrict__ out4) {
+  constexpr int N = Lanes<real>::N, kAhead = 4;
   const int which = blockIdx.y;
   const real* p = which == 0 ? a0 : which == 1 ? a1 : which == 2 ? a2 : a3;
-  const size_t n = which == 0 ? n0 : which == 1 ? n1 : which == 2 ? n2 : n3;
-  double m = 0.0;
+  const size_t quads = (which == 0 ? n0 : which == 1 ? n1 : which == 2 ? n2 : n3) / N;  // rows are whole 16-byte units
+  real big = real(0);
   bool nan = false;
-  for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
-    const double v = fabs((double)p[i]);
-    nan |= (v != v);
-    m = fmax(m, v);
+  const size_t stride = (size_t)gridDim.x * blockDim.x;
+  for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < quads; i += kAhead * stride) {
+    Run<real> v[kAhead];
+#pragma unroll
+    for (int u = 0; u < kAhead; ++u) v[u] = i + u * stride < quads ? ldg16(p + (i + u * stride) * N) : zero_run<real>();
+#pragma unroll
+    for (int u = 0; u < kAhead; ++u)
+#pragma unroll
+      for (int r = 0; r < N; ++r) {
+        const real x = v[u].x[r] < real(0) ? -v[u].x[r] : v[u].x[r];
+        nan |= x != x;
+        big = x > big ? x : big;
+      }
   }
+  const double m = (double)big;
   unsigned long long bits = nan ? 0x7FF8000000000000ull : (unsigned long long)__double_as_longlong(m);
 #pragma unroll
   for (int s = 16; s > 0; s >>= 1) {
