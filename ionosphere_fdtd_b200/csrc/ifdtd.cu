@@ -733,7 +733,7 @@ int build_plan(ifdtd_plan* P, const ifdtd_mesh_desc* M, const ifdtd_grid_desc* G
   if (e_threads_req != 0 &&
       (e_threads_req % 32 || e_threads_req < 32 || e_threads_req + 32 * e_producers > pipe::kWideMaxThreads))
     return fail(IFDTD_ERR_ARGUMENT, "e_threads must be 0 or a multiple of 32 with e_threads + 32 * E producer warps <= 640");
-  if (e_threads_req + 32 * e_producers > pipe::kMaxThreads && staging == 3)
+  if (e_threads_req > 0 && e_threads_req + 32 * e_producers > pipe::kMaxThreads && staging == 3)
     return fail(IFDTD_ERR_ARGUMENT, "wide E-phase CTAs (e_threads + 32 * E producer warps > 384) use TMA bulk copies only");
   const int e_copy_gap = tune ? tune->e_copy_gap : 0;
   if (e_copy_gap < 0 || e_copy_gap > 8) return fail(IFDTD_ERR_ARGUMENT, "e_copy_gap must be 0 to 8");
@@ -1439,7 +1439,11 @@ int build_plan(ifdtd_plan* P, const ifdtd_mesh_desc* M, const ifdtd_grid_desc* G
     // 256 when the count is automatic)
     const int row_quads = std::max(Pn, Pm) / (16 / (int)sizeof(real));
     const bool quads_fit = row_quads <= (auto_threads ? 256 : threads) && (e_threads_req == 0 || row_quads <= e_threads_req);
-    std::vector<int> h_cand = auto_h ? std::vector<int>{256, 128, 64, 32, 16, 8} : std::vector<int>{fpp};
+    // the largest that fits, of sizes whose patches are whole runs of 16-face
+    // subdivision triangles: 48 where 64 does not fit (s6 / 50 cells H 52 us, 60 with
+    // 32), 112 and 96 where 128 does not (s7 / 40 without plasma 72 and 74, 76 with 64);
+    // 80 has more halo for its size (s8 / 60 402 us, 382 with 64)
+    std::vector<int> h_cand = auto_h ? std::vector<int>{256, 128, 112, 96, 64, 48, 32, 16, 8} : std::vector<int>{fpp};
     if (!quads_fit) h_cand.clear();
     for (const int c : h_cand) {
       Own o = ownership(c);
@@ -1574,13 +1578,17 @@ int build_plan(ifdtd_plan* P, const ifdtd_mesh_desc* M, const ifdtd_grid_desc* G
       return fail(IFDTD_ERR_ARGUMENT, "direct kernels take at most 256 threads per CTA");
     if (auto_threads && P->h_mode == 2 && P->e_mode == 2) threads = pipe::kMaxThreads - 32 * producers;
     P->threads = threads;
-    // E-phase compute threads: as given; automatic with automatic threads: the
-    // pipelined CTA's 384 less the E producer warps; otherwise as threads
+    // E-phase compute threads: as given; automatic with automatic threads: what 16
+    // warps leave beside the E producer warps (12 of 12 warps on cp.async copies);
+    // otherwise as threads.  The consumers set the phase's time, and a third more of
+    // them at 128 registers are 2-4 % faster: s8 / 80 cells 752 us (8 consumer warps 770),
+    // s6 / 50 41.1 (43.0), s7 / 40 109.5 (110.7)
+    const bool auto_e_threads = e_threads_req == 0 && auto_threads && P->h_mode == 2 && P->e_mode == 2;
     P->e_threads = e_threads_req > 0 ? e_threads_req
-                   : (auto_threads && P->h_mode == 2 && P->e_mode == 2) ? pipe::kMaxThreads - 32 * e_producers
-                                                                        : threads;
+                   : auto_e_threads  ? (P->pipe_copy == 0 ? pipe::kMidMaxThreads : pipe::kMaxThreads) - 32 * e_producers
+                                     : threads;
     if (P->e_mode == 2 && P->e_threads + 32 * e_producers > pipe::kMaxThreads &&
-        (e_threads_req == 0 || P->pipe_copy != 0))
+        ((e_threads_req == 0 && !auto_e_threads) || P->pipe_copy != 0))
       return fail(IFDTD_ERR_ARGUMENT, "threads + 32 * E producer warps must not exceed 384");
     // rows on 8-lane boundaries only while a rounded-up row still fits the
     // compute threads of both phases (otherwise the rows stay packed)
@@ -1735,9 +1743,10 @@ template <typename real, bool PL, int MD>
 cudaError_t launch_ke_t(ifdtd_plan* P, const Rec<real>* rec, int istep, cudaStream_t st) {
   if (P->e_mode == 2) {
     const int threads = P->e_threads + 32 * P->e_producers;
-    auto k = threads > pipe::kMaxThreads ? pipe::ke_tma<real, PL, MD, 0, pipe::kWideRegs>
-             : P->pipe_copy == 0         ? pipe::ke_tma<real, PL, MD, 0, pipe::kMaxRegs>
-                                         : pipe::ke_tma<real, PL, MD, 1, pipe::kMaxRegs>;
+    auto k = threads > pipe::kMidMaxThreads ? pipe::ke_tma<real, PL, MD, 0, pipe::kWideRegs>
+             : threads > pipe::kMaxThreads  ? pipe::ke_tma<real, PL, MD, 0, pipe::kMidRegs>
+             : P->pipe_copy == 0            ? pipe::ke_tma<real, PL, MD, 0, pipe::kMaxRegs>
+                                            : pipe::ke_tma<real, PL, MD, 1, pipe::kMaxRegs>;
     cudaError_t e = allow_smem_once(P, kLaunchKe, k, P->ke_smem);
     if (e == cudaSuccess) e = persistent_grid(P, k, threads, P->ke_smem, P->n_patches_e, &P->ke_grid);
     if (e != cudaSuccess) return e;
@@ -2136,22 +2145,19 @@ auto batch_kh_kernel(const BatchGroup& g) {
   return g.copy ? kh_tma_batch<real, false, 1> : kh_tma_batch<real, false, 0>;
 }
 
+template <typename real, bool PL, int MD>
+auto batch_ke_kernel_t(const BatchGroup& g) {
+  using namespace pipe;
+  const int threads = g.e_threads + 32 * g.e_producers;
+  return threads > kMidMaxThreads ? ke_tma_batch<real, PL, MD, 0, kWideRegs>
+         : threads > kMaxThreads  ? ke_tma_batch<real, PL, MD, 0, kMidRegs>
+         : g.copy                 ? ke_tma_batch<real, PL, MD, 1, kMaxRegs>
+                                  : ke_tma_batch<real, PL, MD, 0, kMaxRegs>;
+}
 template <typename real>
 auto batch_ke_kernel(const BatchGroup& g) {
-  using namespace pipe;
-  const bool wide = g.e_threads + 32 * g.e_producers > kMaxThreads;
-  if (g.plasma) {
-    if (g.maxdeg == 6)
-      return wide ? ke_tma_batch<real, true, 6, 0, kWideRegs>
-                  : g.copy ? ke_tma_batch<real, true, 6, 1, kMaxRegs> : ke_tma_batch<real, true, 6, 0, kMaxRegs>;
-    return wide ? ke_tma_batch<real, true, 12, 0, kWideRegs>
-                : g.copy ? ke_tma_batch<real, true, 12, 1, kMaxRegs> : ke_tma_batch<real, true, 12, 0, kMaxRegs>;
-  }
-  if (g.maxdeg == 6)
-    return wide ? ke_tma_batch<real, false, 6, 0, kWideRegs>
-                : g.copy ? ke_tma_batch<real, false, 6, 1, kMaxRegs> : ke_tma_batch<real, false, 6, 0, kMaxRegs>;
-  return wide ? ke_tma_batch<real, false, 12, 0, kWideRegs>
-              : g.copy ? ke_tma_batch<real, false, 12, 1, kMaxRegs> : ke_tma_batch<real, false, 12, 0, kMaxRegs>;
+  if (g.plasma) return g.maxdeg == 6 ? batch_ke_kernel_t<real, true, 6>(g) : batch_ke_kernel_t<real, true, 12>(g);
+  return g.maxdeg == 6 ? batch_ke_kernel_t<real, false, 6>(g) : batch_ke_kernel_t<real, false, 12>(g);
 }
 
 template <typename real>
@@ -2201,6 +2207,9 @@ int batch_build(ifdtd_batch* B) {
       key.lanes = P->lanes;
       key.e_threads = P->e_threads;
       key.e_producers = P->e_producers;
+      // the batched E kernel with plasma spills at 128 registers: 8 consumer warps there
+      if (P->plasma && key.e_threads + 32 * key.e_producers == pipe::kMidMaxThreads)
+        key.e_threads = pipe::kMaxThreads - 32 * key.e_producers;
     }
     BatchGroup* g = nullptr;
     for (auto& x : B->groups)

@@ -32,8 +32,11 @@ constexpr int kMaxDesc = 32 * kDescPerLane;  // copy descriptors per patch
 constexpr int kMaxThreads = 384;             // producer warps + compute warps
 // Registers are granted to warps in groups of four: 12 warps x 32 x 168 <= 65536.
 constexpr int kMaxRegs = 168;
-// Wide E-phase CTAs: up to 20 warps at 96 registers (20 x 32 x 96 <= 65536);
-// the E consumer fits 96 registers without spilling, the H consumer does not.
+// E-phase CTAs of up to 16 warps have 128 registers (16 x 32 x 128 = 65536), which
+// the E consumer fits with its layer factors kept; up to 20 warps, 96 registers,
+// where it re-reads them.  The H consumer needs 168.
+constexpr int kMidRegs = 128;
+constexpr int kMidMaxThreads = 512;
 constexpr int kWideRegs = 96;
 constexpr int kWideMaxThreads = 640;
 constexpr uint64_t kWaitNs = 500ull * 1000 * 1000;  // bound of one wait (0.5 s)
@@ -423,8 +426,8 @@ __device__ __forceinline__ void kh_consume(const Rec<real>& R, const Layers<real
 // in registers in the float kernels of vertex degree 6; elsewhere (float64,
 // 12-slot tables) holding them would push the kernel past its register budget
 // into local memory, so they are re-read per run.
-template <typename real, int MAXDEG>
-constexpr bool kHoistVertex = sizeof(real) == 4 && MAXDEG == 6;
+template <typename real, int MAXDEG, int REGS>
+constexpr bool kHoistVertex = sizeof(real) == 4 && MAXDEG == 6 && REGS > kWideRegs;
 template <typename real>
 struct ELanes {
   LaneMap vertex, edge;
@@ -433,7 +436,7 @@ struct ELanes {
   EdgeLayer<real> ey;
   unsigned pattern;  // lanes of this warp that hold a vertex quad
 };
-template <typename real, int MAXDEG>
+template <typename real, int MAXDEG, int REGS>
 __device__ __forceinline__ ELanes<real> e_lanes(const Rec<real>& R, const Layers<real>& Ls, int ct, int nct, int layout) {
   constexpr int N = Lanes<real>::N;
   ELanes<real> m{};
@@ -442,14 +445,14 @@ __device__ __forceinline__ ELanes<real> e_lanes(const Rec<real>& R, const Layers
   m.vertex0 = ct / m.vertex.G;
   m.edge0 = ct / m.edge.G;
   if (!R.coef_full) {
-    if (kHoistVertex<real, MAXDEG> && m.vertex.on) m.vy = vertex_layer(R, Ls, 0, m.vertex.q * N);
-    if (m.edge.on) m.ey = edge_layer(R, Ls, 0, m.edge.q * N);
+    if (kHoistVertex<real, MAXDEG, REGS> && m.vertex.on) m.vy = vertex_layer(R, Ls, 0, m.vertex.q * N);
+    if (REGS > kWideRegs && m.edge.on) m.ey = edge_layer(R, Ls, 0, m.edge.q * N);
   }
   m.pattern = __ballot_sync(0xFFFFFFFFu, m.vertex.on);
   return m;
 }
 
-template <typename real, bool PLASMA, int MAXDEG>
+template <typename real, bool PLASMA, int MAXDEG, int REGS>
 __device__ __forceinline__ void ke_consume(const Rec<real>& R, const Layers<real>& Ls, const ELanes<real>& lanes,
                                            unsigned char* st, int ct, real current) {
   constexpr int N = Lanes<real>::N;
@@ -527,7 +530,7 @@ __device__ __forceinline__ void ke_consume(const Rec<real>& R, const Layers<real
 #pragma unroll
         for (int r = 0; r < N; ++r) rav[r + 1] = own.x[r];
       }
-      e_vertex_run<real, PLASMA, MAXDEG>(R, kHoistVertex<real, MAXDEG> && !full ? lanes.vy : vertex_layer(R, Ls, v, k0),
+      e_vertex_run<real, PLASMA, MAXDEG>(R, kHoistVertex<real, MAXDEG, REGS> && !full ? lanes.vy : vertex_layer(R, Ls, v, k0),
                                          (src & 1) != 0, v, k0, hrows, jrows, vcoef + vl * SW,
                                          PLASMA ? vwc + vl * w_stride : nullptr, s_er + vl * Pn,
                                          R.er + (size_t)v * Pn, current, PLASMA ? rav : nullptr);
@@ -535,10 +538,11 @@ __device__ __forceinline__ void ke_consume(const Rec<real>& R, const Layers<real
   }
   if (lanes.edge.on) {
     const int j0 = lanes.edge.q * N;
+    const EdgeLayer<real> fixed = REGS > kWideRegs ? lanes.ey : edge_layer(R, Ls, ea, j0);
     for (int el = lanes.edge0; el < ne; el += lanes.edge.per) {
       const int e = ea + el;
       const int4 loc = eloc[el];
-      e_edge_run<real, PLASMA>(R, full ? edge_layer(R, Ls, e, j0) : lanes.ey, (src & 2) != 0, e, j0, s_hr + loc.y,
+      e_edge_run<real, PLASMA>(R, full ? edge_layer(R, Ls, e, j0) : fixed, (src & 2) != 0, e, j0, s_hr + loc.y,
                                s_hr + loc.z, s_ht + loc.x, PLASMA ? s_J + loc.y * 3 : nullptr,
                                PLASMA ? s_J + loc.z * 3 : nullptr, s_et + el * Pm, R.et + (size_t)e * Pm, current,
                                einv[el], PLASMA ? etan + el * t_stride : nullptr);
@@ -629,9 +633,9 @@ __global__ void __maxnreg__(REGS) ke_tma(const Rec<real>* __restrict__ recs, int
     Layers<real> Ls;
     consumer_layers(R, dyn_smem, Ls, ct, nct);
     const real current = (R.n_src_er + R.n_src_et) > 0 ? (real)R.cur[istep] : real(0);
-    const ELanes<real> lanes = e_lanes<real, MAXDEG>(R, Ls, ct, nct, layout);
+    const ELanes<real> lanes = e_lanes<real, MAXDEG, REGS>(R, Ls, ct, nct, layout);
     consume_ring(G, p0, p1, [&](unsigned char* st, int s, uint32_t ph) {
-      ke_consume<real, PLASMA, MAXDEG>(R, Ls, lanes, st, ct, current);
+      ke_consume<real, PLASMA, MAXDEG, REGS>(R, Ls, lanes, st, ct, current);
     });
   }
 }
@@ -720,9 +724,9 @@ __global__ void __maxnreg__(REGS) ke_tma_batch(const Rec<real>* __restrict__ rec
       Layers<real> Ls;
       consumer_layers(R, dyn_smem, Ls, ct, nct);
       const real current = (R.n_src_er + R.n_src_et) > 0 ? (real)R.cur[istep] : real(0);
-      const ELanes<real> lanes = e_lanes<real, MAXDEG>(R, Ls, ct, nct, layout);
+      const ELanes<real> lanes = e_lanes<real, MAXDEG, REGS>(R, Ls, ct, nct, layout);
       consume_ring(G, sg.y, sg.z, [&](unsigned char* st, int s, uint32_t ph) {
-        ke_consume<real, PLASMA, MAXDEG>(R, Ls, lanes, st, ct, current);
+        ke_consume<real, PLASMA, MAXDEG, REGS>(R, Ls, lanes, st, ct, current);
       });
     }
   }
