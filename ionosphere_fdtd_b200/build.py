@@ -23,6 +23,7 @@ HEADERS = [
     PACKAGE / "csrc" / "fused_kernels.cuh",
     PACKAGE / "csrc" / "loop_kernels.cuh",
     PACKAGE / "csrc" / "errors.cuh",
+    PACKAGE / "csrc" / "launch.cuh",
     PACKAGE / "csrc" / "silu.cuh",
     PACKAGE / "csrc" / "tc_common.cuh",
     ROOT / "include" / "ifdtd.h",

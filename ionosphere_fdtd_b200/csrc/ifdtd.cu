@@ -1729,7 +1729,7 @@ cudaError_t launch_kh_t(ifdtd_plan* P, const Rec<real>* rec, cudaStream_t st) {
     cudaError_t e = allow_smem_once(P, kLaunchKh, k, P->kh_smem);
     if (e == cudaSuccess) e = persistent_grid(P, k, threads, P->kh_smem, P->n_patches, &P->kh_grid);
     if (e != cudaSuccess) return e;
-    k<<<P->kh_grid, threads, P->kh_smem, st>>>(rec, P->kh_stage, P->kh_stages, P->producers, P->lanes);
+    return launch_after(k, P->kh_grid, threads, P->kh_smem, st, rec, P->kh_stage, P->kh_stages, P->producers, P->lanes);
   } else {
     auto k = kh_kernel<real, PL>;
     cudaError_t e = allow_smem_once(P, kLaunchKh, k, P->smem_bytes);
@@ -1750,7 +1750,8 @@ cudaError_t launch_ke_t(ifdtd_plan* P, const Rec<real>* rec, int istep, cudaStre
     cudaError_t e = allow_smem_once(P, kLaunchKe, k, P->ke_smem);
     if (e == cudaSuccess) e = persistent_grid(P, k, threads, P->ke_smem, P->n_patches_e, &P->ke_grid);
     if (e != cudaSuccess) return e;
-    k<<<P->ke_grid, threads, P->ke_smem, st>>>(rec, P->ke_stage, P->ke_stages, P->e_producers, istep, P->lanes);
+    return launch_after(k, P->ke_grid, threads, P->ke_smem, st, rec, P->ke_stage, P->ke_stages, P->e_producers, istep,
+                        P->lanes);
   } else {
     auto k = ke_kernel<real, PL, MD>;
     cudaError_t e = allow_smem_once(P, kLaunchKe, k, P->smem_bytes);
@@ -1841,8 +1842,8 @@ cudaError_t launch_step(ifdtd_plan* P, int istep, int blocks, int row, cudaStrea
     if (e == cudaSuccess) e = launch_ke<real>(P, istep, st);
   }
   if (e != cudaSuccess) return e;
-  if (blocks > 0) sample_slots_kernel<real><<<blocks, 256, 0, st>>>(rec, P->d_slots, row);
-  return cudaGetLastError();
+  if (blocks > 0) return launch_after(sample_slots_kernel<real>, blocks, 256, 0, st, rec, P->d_slots, row);
+  return cudaSuccess;
 }
 
 // Face frames: the caller's Cartesian plasma currents turned into the plan's
@@ -2319,9 +2320,8 @@ cudaError_t batch_launch_step(ifdtd_batch* B, int istep, int rows, int step_row,
     const BatchGroup& g = B->groups[q];
     if (g.fused) continue;
     auto k = batch_kh_kernel<real>(g);
-    k<<<g.kh_grid, g.threads + 32 * g.producers, g.kh_smem, st>>>(recs, g.segs_h, g.sptr_h, B->d_ring_h, g.producers,
-                                                                   g.lanes);
-    e = cudaGetLastError();
+    e = launch_after(k, g.kh_grid, g.threads + 32 * g.producers, g.kh_smem, st, recs, g.segs_h, g.sptr_h, B->d_ring_h,
+                     g.producers, g.lanes);
     if (e != cudaSuccess) B->failed = "kh_tma_batch of group " + std::to_string(q);
   }
   for (size_t q = 0; q < B->solo.size() && e == cudaSuccess; ++q) {
@@ -2332,9 +2332,8 @@ cudaError_t batch_launch_step(ifdtd_batch* B, int istep, int rows, int step_row,
     const BatchGroup& g = B->groups[q];
     if (g.fused) continue;
     auto k = batch_ke_kernel<real>(g);
-    k<<<g.ke_grid, g.e_threads + 32 * g.e_producers, g.ke_smem, st>>>(recs, g.segs_e, g.sptr_e, B->d_ring_e, g.e_producers,
-                                                                   istep, g.lanes);
-    e = cudaGetLastError();
+    e = launch_after(k, g.ke_grid, g.e_threads + 32 * g.e_producers, g.ke_smem, st, recs, g.segs_e, g.sptr_e, B->d_ring_e,
+                     g.e_producers, istep, g.lanes);
     if (e != cudaSuccess) B->failed = "ke_tma_batch of group " + std::to_string(q);
   }
   for (size_t q = 0; q < B->solo.size() && e == cudaSuccess; ++q) {
@@ -2344,9 +2343,8 @@ cudaError_t batch_launch_step(ifdtd_batch* B, int istep, int rows, int step_row,
   if (rows > 0 && e == cudaSuccess) {
     // after a parity-0 step the fused members' state is in their second copies
     const Rec<real>* now = B->any_fused && !parity ? recs_b : recs;
-    sample_batch_kernel<real><<<(rows * 32 + 255) / 256, 256, 0, st>>>(now, (const ProbeRef*)B->d_refs,
-                                                                         (const int2*)B->d_rowmap, rows, step_row);
-    e = cudaGetLastError();
+    e = launch_after(sample_batch_kernel<real>, (rows * 32 + 255) / 256, 256, 0, st, now, (const ProbeRef*)B->d_refs,
+                     (const int2*)B->d_rowmap, rows, step_row);
     if (e != cudaSuccess) B->failed = "sample_batch_kernel";
   }
   return e;

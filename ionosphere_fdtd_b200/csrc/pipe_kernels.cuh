@@ -587,9 +587,15 @@ __device__ __forceinline__ void consumer_layers(const Rec<real>& R, unsigned cha
   asm volatile("bar.sync 1, %0;" ::"r"(nct) : "memory");
 }
 
+// The phases follow one another with programmatic dependence (launch.cuh): while the
+// launch before drains, a CTA sets up its record, barriers, layer rows and lane maps,
+// none of which a step writes, and it waits before its first copy or store.  What lay
+// between two launches was 1-2 us: a step at s6 / 50 cells 84.0 -> 81.2 us, s7 / 40
+// 225.3 -> 222.3, s6 / 40 without plasma 31.6 -> 30.1, float64 s5 / 40 35.0 -> 33.2.
 template <typename real, bool PLASMA, int COPY>
 __global__ void __maxnreg__(kMaxRegs) kh_tma(const Rec<real>* __restrict__ recs, int stage_bytes, int n_stages,
                                              int producers, int layout) {
+  launch_next();
   extern __shared__ __align__(128) unsigned char dyn_smem[];
   __shared__ Rec<real> R;
   __shared__ __align__(8) uint64_t full[kMaxStages], empty[kMaxStages], group[kMaxStages];
@@ -602,12 +608,14 @@ __global__ void __maxnreg__(kMaxRegs) kh_tma(const Rec<real>* __restrict__ recs,
   const int n = R.n_patches_h;
   const int p0 = (int)((long long)n * blockIdx.x / gridDim.x), p1 = (int)((long long)n * (blockIdx.x + 1) / gridDim.x);
   if (threadIdx.x < 32 * W) {
+    wait_previous();
     produce<COPY>(R, G, p0, p1, n, R.dptr_h, R.desc_h, threadIdx.x / 32, W);
   } else {
     const int ct = threadIdx.x - 32 * W, nct = blockDim.x - 32 * W;
     Layers<real> Ls;
     consumer_layers(R, dyn_smem, Ls, ct, nct);
     const HLanes<real> lanes = h_lanes(R, Ls, ct, nct, layout);
+    wait_previous();
     consume_ring(G, p0, p1, [&](unsigned char* st, int s, uint32_t ph) {
       kh_consume<real, PLASMA>(R, Ls, lanes, st, ct, nct, group + s, ph, G);
     });
@@ -617,6 +625,7 @@ __global__ void __maxnreg__(kMaxRegs) kh_tma(const Rec<real>* __restrict__ recs,
 template <typename real, bool PLASMA, int MAXDEG, int COPY, int REGS>
 __global__ void __maxnreg__(REGS) ke_tma(const Rec<real>* __restrict__ recs, int stage_bytes, int n_stages,
                                          int producers, int istep, int layout) {
+  launch_next();
   extern __shared__ __align__(128) unsigned char dyn_smem[];
   __shared__ Rec<real> R;
   __shared__ __align__(8) uint64_t full[kMaxStages], empty[kMaxStages];
@@ -627,6 +636,7 @@ __global__ void __maxnreg__(REGS) ke_tma(const Rec<real>* __restrict__ recs, int
   const int n = R.n_patches_e;
   const int p0 = (int)((long long)n * blockIdx.x / gridDim.x), p1 = (int)((long long)n * (blockIdx.x + 1) / gridDim.x);
   if (threadIdx.x < 32 * W) {
+    wait_previous();
     produce<COPY>(R, G, p0, p1, n, R.dptr_e, R.desc_e, threadIdx.x / 32, W);
   } else {
     const int ct = threadIdx.x - 32 * W, nct = blockDim.x - 32 * W;
@@ -634,6 +644,7 @@ __global__ void __maxnreg__(REGS) ke_tma(const Rec<real>* __restrict__ recs, int
     consumer_layers(R, dyn_smem, Ls, ct, nct);
     const real current = (R.n_src_er + R.n_src_et) > 0 ? (real)R.cur[istep] : real(0);
     const ELanes<real> lanes = e_lanes<real, MAXDEG, REGS>(R, Ls, ct, nct, layout);
+    wait_previous();
     consume_ring(G, p0, p1, [&](unsigned char* st, int s, uint32_t ph) {
       ke_consume<real, PLASMA, MAXDEG, REGS>(R, Ls, lanes, st, ct, current);
     });
@@ -671,6 +682,8 @@ __global__ void __maxnreg__(kMaxRegs) kh_tma_batch(const Rec<real>* __restrict__
   __shared__ Rec<real> R;
   __shared__ __align__(8) uint64_t full[kMaxStages], empty[kMaxStages], group[kMaxStages];
   __shared__ int abort_flag;
+  launch_next();
+  wait_previous();
   const int W = producers;
   if (threadIdx.x == 0) abort_flag = 0;
   int prev = 0;
@@ -705,6 +718,8 @@ __global__ void __maxnreg__(REGS) ke_tma_batch(const Rec<real>* __restrict__ rec
   __shared__ Rec<real> R;
   __shared__ __align__(8) uint64_t full[kMaxStages], empty[kMaxStages], group[kMaxStages];
   __shared__ int abort_flag;
+  launch_next();
+  wait_previous();
   const int W = producers;
   if (threadIdx.x == 0) abort_flag = 0;
   int prev = 0;

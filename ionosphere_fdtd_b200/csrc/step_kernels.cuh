@@ -34,6 +34,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include "launch.cuh"
+
 namespace ifdtd {
 
 constexpr int kMaxSpecies = 4;
@@ -1043,6 +1045,8 @@ __device__ __forceinline__ void sample_row(const Rec<real>& R, const SampleSlot&
 // probes nor the fields, so one graph serves every recorded run of its plan.
 template <typename real>
 __global__ void sample_slots_kernel(const Rec<real>* __restrict__ rec, const SampleSlot* __restrict__ slots, int sample) {
+  launch_next();
+  wait_previous();
   const int warps = gridDim.x * (blockDim.x >> 5);
   for (int w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; w < slots[0].rows + slots[1].rows; w += warps) {
     const int first = slots[0].rows;
@@ -1068,6 +1072,8 @@ struct ProbeRef {
 template <typename real>
 __global__ void sample_batch_kernel(const Rec<real>* __restrict__ recs, const ProbeRef* __restrict__ refs,
                                     const int2* __restrict__ rowmap, int total_rows, int step_row) {
+  launch_next();
+  wait_previous();
   const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int lane = threadIdx.x & 31;
   if (warp >= total_rows) return;

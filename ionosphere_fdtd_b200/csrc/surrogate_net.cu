@@ -24,6 +24,7 @@
 
 #include "../../include/ifdtd_surrogate.h"
 #include "errors.cuh"
+#include "launch.cuh"
 #include "silu.cuh"
 #include "tc_common.cuh"
 
@@ -125,12 +126,6 @@ __device__ __forceinline__ void get16(const float* p, float (&v)[16], int n, boo
     for (int q = 0; q < 16; ++q) v[q] = q < n ? __ldg(p + q) : 0.f;
   }
 }
-
-// The launches of a pass follow one another with programmatic dependence: a
-// kernel sets up its barriers, tensor memory and tensor maps while the one before
-// drains, and touches memory only after this wait for all of it.
-__device__ __forceinline__ void launch_next() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
-__device__ __forceinline__ void wait_previous() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
 // One output tile (and split) per CTA of 256 threads.  Thread 0 streams the K
 // chunks through the stage ring (all of them at once where they fit), issues the
@@ -530,22 +525,6 @@ int failed_launch(const char* what, cudaError_t e) {
   return record_error(IFDTD_ERR_CUDA, std::string(what) + ": " + cudaGetErrorString(e));
 }
 
-// A launch that may begin while the one before it on the stream drains (its kernel waits for it).
-template <typename... Args>
-cudaError_t launch_after(void (*kernel)(Args...), int blocks, int threads, size_t smem, cudaStream_t st, const Args&... args) {
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(blocks);
-  cfg.blockDim = dim3(threads);
-  cfg.dynamicSmemBytes = smem;
-  cfg.stream = st;
-  cudaLaunchAttribute at[1];
-  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  at[0].val.programmaticStreamSerializationAllowed = 1;
-  cfg.attrs = at;
-  cfg.numAttrs = 1;
-  return cudaLaunchKernelEx(&cfg, kernel, args...);
-}
-
 int pitch8(int cols) { return (cols + 7) / 8 * 8; }
 
 // Fill the shape of a job.  a, b: bf16 matrices as they lie in memory, lda / ldb
@@ -636,6 +615,7 @@ cudaError_t net_status(int reset, int* out) {
 }  // namespace tc
 }  // namespace ifdtd
 
+using namespace ifdtd;
 using namespace ifdtd::tc;
 
 extern "C" {
