@@ -1605,21 +1605,25 @@ int build_plan(ifdtd_plan* P, const ifdtd_mesh_desc* M, const ifdtd_grid_desc* G
   }
   R.dtmu = (real)(G->time_step_s / 1.256637062120e-6);
   // Steps in one cooperative launch while the whole grid takes a phase's runs in
-  // a few rounds and the launch geometry is automatic.  The line lies where it
+  // a few rounds and the launch geometry is automatic.  The lines lie where it
   // stops being faster than graph-replayed ring launches, us per step, loop
-  // against ring (no receivers, which cost the ring another 2-4 us):
-  //   s2 / 24 cells (0.05 rounds) 5.2 / 12.9; s5 / 37 (4.7) 13.2 / 17.9;
-  //   s6 / 20 (10.5) 22.4 / 27.0; s6 / 26 (13.2) 27.4 / 29.6; s6 / 34 (16.9) 36.7 / 34.4;
-  //   Drude plasma s5 / 40 (7.6) 21.0 / 26.0; magnetised s5 / 50 (9.4) 55.7 / 65.4;
-  //   float64 s5 / 30 (11.5) 17.9 / 19.9.
-  // With a surface impedance one thread walks an edge's poles, so the line lies
-  // lower: s4 / 31 (2.1 rounds) 7.6 / 15.1; plasma s5 / 20 (4.1) 19.4 / 22.4, s5 / 40
-  // (7.6) 29.2 / 29.1.
+  // against ring (no receivers, which cost the ring another 2 us):
+  //   6 rounds: s2 / 24 cells (0.05 rounds) 5.0 / 9.2; s5 / 24 (3.1) 10.7 / 12.2; s5 / 37 (4.7) 13.4 / 14.1; s5 / 46 (5.6)
+  //   14.1 / 14.1; s5 / 60 (7.3) 16.2 / 15.1; Drude plasma s5 / 24 (4.8) 15.3 / 19.2, s5 / 40 (7.6)
+  //   20.8 / 20.0; float64 s5 / 10 (4.3) 10.4 / 11.1, s5 / 30 (11.5) 19.5 / 15.1.
+  //   10 with a magnetised plasma, whose runs are long: s5 / 33 (6.5) 37.8 / 41.2, s5 / 50 (9.4)
+  //   54.5 / 59.0, s5 / 60 (11.2) 67.0 / 60.6; and with rows of up to four runs, of which the
+  //   ring stages many: s6 / 14 (7.5) 17.1 / 18.0, Drude s6 / 10 (8.7) 26.6 / 37.2.
+  //   4 with a surface impedance, where one thread walks an edge's poles: s5 / 20 (2.6) 13.9 /
+  //   14.5, s5 / 37 (4.7) 18.8 / 15.5; Drude s5 / 16 (3.3) 17.0 / 19.7, s5 / 24 (4.8) 20.6 / 19.9.
   const bool auto_geometry =
       !tune || (auto_h && auto_e && auto_threads && staging == 0 && !fused && e_threads_req == 0 && e_stages_req == 0 &&
                 (tune->producer_warps <= 0 || tune->producer_warps == 2) && tune->e_producer_warps <= 0 &&
                 e_copy_gap == 0 && lane_layout == 0);
-  if (auto_geometry && P->chunk > 0 && loop_rounds<real>(P) <= (X->si_terms > 0 ? 7 : 12)) {
+  const int loop_limit = X->si_terms > 0                                                  ? 4
+                         : X->plasma_magnetized || Pm / (int)(16 / sizeof(real)) <= 4 ? 10
+                                                                                          : 6;
+  if (auto_geometry && P->chunk > 0 && loop_rounds<real>(P) <= loop_limit) {
     P->loop = true;
     void* at = nullptr;
     cudaError_t e = A.alloc(sizeof(unsigned long long), &at);

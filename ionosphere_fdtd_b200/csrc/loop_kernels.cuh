@@ -8,8 +8,8 @@
 // latency: a phase is the barrier (one atomic add per CTA, then polling), one
 // trip to L2 for a run's table entries and one for its rows.  What this saves
 // against a launch per phase is the launch, the record, the layer rows and, for
-// the ring kernels, the descriptors and the staging: 5.2 us per step at s2 / 24
-// cells against 12.9 us of ring launches in a graph, 13.2 against 17.9 at s5 / 37.
+// the ring kernels, the descriptors and the staging: 5.0 us per step at s2 / 24
+// cells against 9.2 us of ring launches in a graph, 13.2 against 14.1 at s5 / 37.
 // The next run's table entries are read before the current run's rows are used
 // (and before the barrier for a phase's first run), and a block has only as many
 // threads as its runs need: 5.6 without either at s2 / 24, 14.6 at s5 / 37.
