@@ -112,17 +112,21 @@ typedef struct ifdtd_physics_desc {
 /* Tuning of the launch geometry (0 = defaults). */
 typedef struct ifdtd_tuning {
   int32_t faces_per_patch;   /* faces owned by one H-phase patch (0: fit the pipeline stage to shared memory) */
-  int32_t threads;           /* threads per direct CTA, or compute threads per pipelined CTA (0: automatic) */
-  int32_t graph_chunk;       /* steps captured per CUDA graph (default 32; 0 disables) */
+  int32_t threads;           /* threads per direct CTA, or compute threads per pipelined CTA (0: 256 direct, 384 less
+                                the copy warps pipelined) */
+  int32_t graph_chunk;       /* steps captured per CUDA graph (default 32; 0: none, and no loop kernel) */
   int32_t e_faces_per_patch; /* faces whose vertices/edges one E-phase patch owns (0: fit the stage to shared memory) */
-  int32_t staging;           /* 0 auto, 1 direct global gathers, 2 pipeline (TMA bulk copies), 3 pipeline (cp.async) */
+  int32_t staging;           /* 0 auto (small plans with every geometry field automatic: many steps in one
+                                cooperative launch), 1 direct global gathers, 2 pipeline (TMA bulk copies),
+                                3 pipeline (cp.async) */
   int32_t producer_warps;    /* copy-issuing warps per pipelined CTA (default 2, at most 4) */
   int32_t lane_layout;       /* pipelined consumers: 0 auto (packed), 1 rows packed back to back across lanes,
                                 2 every row starting on an 8-lane boundary (no shared-memory bank conflicts
                                 between rows; rows stay packed when a rounded-up row exceeds the threads) */
-  int32_t e_threads;         /* compute threads of a pipelined E-phase CTA (0: as threads); with the producer
-                                warps above 384 the E phase runs wide CTAs at 96 registers (at most 640
-                                threads, TMA bulk copies only) */
+  int32_t e_threads;         /* compute threads of a pipelined E-phase CTA (0: 512 less the copy warps when
+                                threads is automatic too, else as threads); with the copy warps up to 384
+                                threads have 168 registers, up to 512 128 and up to 640 96 (above 384 TMA
+                                bulk copies only) */
   int32_t e_stages;          /* E-phase ring stages the balanced patches are sized for (0: 2, else 2 to 4) */
   int32_t e_producer_warps;  /* copy-issuing warps of a pipelined E-phase CTA (0: 4 when threads and e_threads
                                 are automatic, else as producer_warps; or 1 to 4) */

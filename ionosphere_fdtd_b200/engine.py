@@ -40,14 +40,16 @@ class Tuning:
     per CTA (direct kernels, at most 256) or compute threads per CTA besides
     the producer warps (pipelined kernels; 0: 256 direct, 384 - 32 x producer
     warps pipelined), steps per captured
-    CUDA graph, and the kernel family (0 auto: the pipeline wherever two patch
-    stages fit in shared memory, 1 direct global gathers, 2 the warp-specialised
+    CUDA graph (0: none, and no loop kernel either), and the kernel family (0 auto: small plans whose geometry
+    is all automatic run many steps in one cooperative launch of the loop kernel,
+    others the pipeline wherever two patch stages fit in shared memory, 1 direct global gathers, 2 the warp-specialised
     pipeline fed by TMA bulk copies, 3 the same pipeline fed by 16-byte cp.async
     copies), the copy-issuing warps per pipelined CTA (1 to 4), and the lane
     layout of the pipelined consumers (0 auto = 1, rows packed back to back
     across lanes; 2, every row starting on an 8-lane boundary), the compute
-    threads of an E-phase CTA (0: as ``threads``; above 384 minus the producer
-    warps the E phase runs wide CTAs of at most 640 threads at 96 registers)
+    threads of an E-phase CTA (0: 512 minus the producer warps when ``threads``
+    is automatic too, else as ``threads``; with the producer warps up to 384
+    threads have 168 registers, up to 512 128, up to 640 96),
     the ring stages the balanced E patches are sized for (0: 2), the
     copy-issuing warps of an E-phase CTA (0: 4 when both thread counts are
     automatic, else as ``producer_warps``), the

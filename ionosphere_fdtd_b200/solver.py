@@ -5,9 +5,9 @@ Drop-in for the reference's ``GeodesicFDTD`` on its PyTorch CUDA backend
 validation messages, ``step()``, observation recording, ``diagnostics()`` and
 checkpoint layout.  The host does exactly the reference's setup (material
 sampling, CFL limit, loss coefficients, source supports, ADE coefficients)
-and hands it to a native plan; every time step then runs as two fused CUDA
-launches (H phase, E phase) on torch's current stream, replayed from CUDA
-graphs in chunks.  There is no CPU fallback: without a CUDA device the
+and hands it to a native plan, which runs on torch's current stream: on small
+meshes many time steps in one cooperative launch, elsewhere two launches per step
+(H phase, E phase), replayed from CUDA graphs in chunks.  There is no CPU fallback: without a CUDA device the
 constructor raises ``BackendUnavailableError``.
 """
 
