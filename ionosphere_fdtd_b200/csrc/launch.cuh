@@ -4,7 +4,9 @@
 // an earlier launch may still write or read; the wait is for the whole of the kernel
 // before, which in its turn waited for the one before it.  launch_next allows the
 // following launch_after to begin; a plain launch or copy that follows still waits
-// for the end of the kernel.
+// for the end of the kernel.  A kernel calls launch_next only when it holds all that it
+// may have to wait for and that the following kernel could take first (tensor memory):
+// what the following kernel holds, it holds until this one has ended.
 #pragma once
 
 #include <cuda_runtime.h>

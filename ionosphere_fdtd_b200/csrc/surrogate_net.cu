@@ -132,8 +132,14 @@ __device__ __forceinline__ void get16(const float* p, float (&v)[16], int n, boo
 // MMAs of chunk c into accumulator c / kps and commits them to the stage; then
 // warps w and w + 4 read the TMEM lanes 32 (w % 4) .. + 31, alternate groups of 16
 // columns each, and run the epilogue, whose other operands were loaded meanwhile.
-// Every wait is bounded; a wait that runs out sets the status bit and the CTA
-// skips its epilogue after its own copies and MMAs have ended.
+// Every mbarrier wait is bounded; one that runs out sets the status bit and the CTA
+// skips its epilogue after its own copies and MMAs have ended.  Two waits have no
+// bound: tcgen05.alloc, while other CTAs of the SM hold the columns, and
+// wait_previous, for the end of the launch before.  A CTA therefore lets the next
+// launch begin only once its own columns are allocated: a CTA of the next launch may
+// hold columns in wait_previous, and if this launch still needed them, neither would
+// go on.  With that order a launch never waits for one that follows it, and CTAs of
+// the same launch that wait for each other's columns end one after the other.
 __global__ void __launch_bounds__(LTHREADS) layer_gemm(const __grid_constant__ Launch L) {
   extern __shared__ unsigned char smem_raw[];
   __shared__ __align__(8) uint64_t full[kMaxLayerStages], empty[kMaxLayerStages], done;
@@ -141,7 +147,6 @@ __global__ void __launch_bounds__(LTHREADS) layer_gemm(const __grid_constant__ L
   __shared__ uint32_t tmem_slot;
   __shared__ int failed;
   unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
-  launch_next();
   const bool second = (int)blockIdx.x >= L.first_of_second;
   const Job& J = L.job[second ? 1 : 0];
   int t = (int)blockIdx.x - (second ? L.first_of_second : 0);
@@ -158,6 +163,8 @@ __global__ void __launch_bounds__(LTHREADS) layer_gemm(const __grid_constant__ L
                  : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
   }
+  __syncthreads();
+  launch_next();
   auto load = [&](int c) {
     const int s = c % J.stages;
     const uint32_t as = smem_u32(smem + s * J.stage_bytes), bs = as + LA_BYTES, bar = smem_u32(&full[s]);
