@@ -103,6 +103,7 @@ struct ifdtd_plan {
   int producers = 2;           // copy-issuing warps per pipelined CTA
   int lanes = 0;               // lane layout of the pipelined consumers: 0 packed rows, 1 rows on 8-lane boundaries
   int e_threads = 0;           // compute threads of a pipelined E-phase CTA (above 384 - 32 x e_producers: wide CTAs)
+  bool e_threads_auto = false;  // chosen here, not asked for
   int e_producers = 2;         // copy-issuing warps of a pipelined E-phase CTA
   bool pipe_h_ok = false, pipe_e_ok = false;
   int kh_stage = 0, ke_stage = 0, kh_stages = 0, ke_stages = 0, kh_grid = 0, ke_grid = 0, sm_count = 148;
@@ -1584,6 +1585,7 @@ int build_plan(ifdtd_plan* P, const ifdtd_mesh_desc* M, const ifdtd_grid_desc* G
     // them at 128 registers are 2-4 % faster: s8 / 80 cells 752 us (8 consumer warps 770),
     // s6 / 50 41.1 (43.0), s7 / 40 109.5 (110.7)
     const bool auto_e_threads = e_threads_req == 0 && auto_threads && P->h_mode == 2 && P->e_mode == 2;
+    P->e_threads_auto = auto_e_threads;
     P->e_threads = e_threads_req > 0 ? e_threads_req
                    : auto_e_threads  ? (P->pipe_copy == 0 ? pipe::kMidMaxThreads : pipe::kMaxThreads) - 32 * e_producers
                                      : threads;
@@ -2154,8 +2156,10 @@ template <typename real, bool PL, int MD>
 auto batch_ke_kernel_t(const BatchGroup& g) {
   using namespace pipe;
   const int threads = g.e_threads + 32 * g.e_producers;
+  // with plasma the batched kernel spills at 128 registers and fits 96, where it re-reads its layer factors
+  constexpr int kMid = PL ? kWideRegs : kMidRegs;
   return threads > kMidMaxThreads ? ke_tma_batch<real, PL, MD, 0, kWideRegs>
-         : threads > kMaxThreads  ? ke_tma_batch<real, PL, MD, 0, kMidRegs>
+         : threads > kMaxThreads  ? ke_tma_batch<real, PL, MD, 0, kMid>
          : g.copy                 ? ke_tma_batch<real, PL, MD, 1, kMaxRegs>
                                   : ke_tma_batch<real, PL, MD, 0, kMaxRegs>;
 }
@@ -2212,8 +2216,9 @@ int batch_build(ifdtd_batch* B) {
       key.lanes = P->lanes;
       key.e_threads = P->e_threads;
       key.e_producers = P->e_producers;
-      // the batched E kernel with plasma spills at 128 registers: 8 consumer warps there
-      if (P->plasma && key.e_threads + 32 * key.e_producers == pipe::kMidMaxThreads)
+      // the batched E kernel with plasma spills at 128 registers: 8 consumer warps where the count is
+      // automatic (rows then have at most 256 quads), the count asked for otherwise
+      if (P->plasma && P->e_threads_auto && key.e_threads + 32 * key.e_producers == pipe::kMidMaxThreads)
         key.e_threads = pipe::kMaxThreads - 32 * key.e_producers;
     }
     BatchGroup* g = nullptr;
