@@ -136,7 +136,7 @@ struct ifdtd_plan {
   // makes and destroys its probes; at most kSpareBytes are kept)
   void* spare = nullptr;
   size_t spare_bytes = 0;
-  SampleSlot* d_slots = nullptr;  // the run's probes as the sampling launches read them
+  SampleSlot* d_slots = nullptr;  // the run's probes as the sampling launches of the plan's graphs read them
   double* d_samples = nullptr;    // (graph_chunk, rows) of each slot
   size_t sample_values = 0;
   unsigned opted = 0;  // launch kinds whose shared-memory limit is raised
@@ -1834,9 +1834,15 @@ cudaError_t launch_fused(ifdtd_plan* P, int istep, int parity, cudaStream_t st) 
   return cudaGetLastError();
 }
 
-// One step; with blocks > 0 its state is sampled into row `row` of the plan's slots.
+// Sampling at the end of a step: its blocks (0: none), the row written, and the
+// slots by value (null: the plan's slots, in its own graphs).
+struct Sampling {
+  int blocks = 0, row = 0;
+  const SampleSlots* now = nullptr;
+};
+
 template <typename real>
-cudaError_t launch_step(ifdtd_plan* P, int istep, int blocks, int row, cudaStream_t st, int parity = 0) {
+cudaError_t launch_step(ifdtd_plan* P, int istep, const Sampling& sampling, cudaStream_t st, int parity = 0) {
   const Rec<real>* rec = (const Rec<real>*)P->d_rec;
   cudaError_t e;
   if (P->fused) {
@@ -1848,8 +1854,10 @@ cudaError_t launch_step(ifdtd_plan* P, int istep, int blocks, int row, cudaStrea
     if (e == cudaSuccess) e = launch_ke<real>(P, istep, st);
   }
   if (e != cudaSuccess) return e;
-  if (blocks > 0) return launch_after(sample_slots_kernel<real>, blocks, 256, 0, st, rec, P->d_slots, row);
-  return cudaSuccess;
+  const int blocks = sampling.blocks, row = sampling.row;
+  if (blocks <= 0) return cudaSuccess;
+  return sampling.now ? launch_after(sample_now_kernel<real>, blocks, 256, 0, st, rec, *sampling.now, row)
+                      : launch_after(sample_slots_kernel<real>, blocks, 256, 0, st, rec, P->d_slots, row);
 }
 
 // Face frames: the caller's Cartesian plasma currents turned into the plan's
@@ -1891,12 +1899,19 @@ void fill_slot(SampleSlot& s, const ifdtd_probe* p, double* out) {
 template <typename real>
 int run_launched(ifdtd_plan* P, const double* currents, int n, const Record* rec, int& parity, cudaStream_t stream) {
   const int cap = std::max(P->chunk, 1);
-  // blocks of a sampling launch (8 rows each): powers of two, so a plan keeps few graphs
-  const int rows = rec ? rec->rows() : 0;
+  // Sampled chunks replay the plan's own graphs, whose slots and rows belong to the plan
+  // and whose slots are copied from the host: both are for this call alone.  A caller's
+  // capture never holds them (it refuses graph launches), only launches that carry their
+  // slots and write the caller's rows.
+  const bool graphs = P->chunk > 0 && n >= cap;
+  // blocks of a sampling launch (8 rows each); in a graph powers of two, so a plan keeps few graphs
+  const int rows = rec ? rec->rows() : 0, now_blocks = (rows + 7) / 8;
   int blocks = rec ? 1 : 0;
   while (blocks && blocks < 64 && 8 * blocks < rows) blocks *= 2;
+  SampleSlots now = {};
+  for (int q = 0; rec && q < rec->n; ++q) fill_slot(now.slot[q], rec->probe[q], rec->out[q]);
   size_t offset[kMaxSlots] = {0, 0};
-  if (rec) {
+  if (rec && graphs) {
     if ((size_t)cap * rows > P->sample_values) {
       CUDA_TRY(cudaStreamSynchronize(stream));
       cudaFree(P->d_samples);
@@ -1905,13 +1920,13 @@ int run_launched(ifdtd_plan* P, const double* currents, int n, const Record* rec
       CUDA_TRY(cudaMalloc((void**)&P->d_samples, (size_t)cap * rows * sizeof(double)));
       P->sample_values = (size_t)cap * rows;
     }
-    SampleSlot slots[kMaxSlots] = {};
+    SampleSlots slots = now;
     for (int q = 0; q < rec->n; ++q) {
       offset[q] = q ? (size_t)cap * rec->probe[0]->rows : 0;
-      fill_slot(slots[q], rec->probe[q], P->d_samples + offset[q]);
+      slots.slot[q].out = P->d_samples + offset[q];
     }
     // pageable source: the runtime stages it before returning
-    CUDA_TRY(cudaMemcpyAsync(P->d_slots, slots, sizeof(slots), cudaMemcpyHostToDevice, stream));
+    CUDA_TRY(cudaMemcpyAsync(P->d_slots, &slots, sizeof(slots), cudaMemcpyHostToDevice, stream));
   }
   for (int s0 = 0; s0 < n; s0 += cap) {
     const int c = std::min(cap, n - s0);
@@ -1919,7 +1934,7 @@ int run_launched(ifdtd_plan* P, const double* currents, int n, const Record* rec
       CUDA_TRY(cudaMemcpyAsync(P->d_cur, currents + s0, c * sizeof(double), cudaMemcpyDeviceToDevice, stream));
     else
       CUDA_TRY(cudaMemsetAsync(P->d_cur, 0, c * sizeof(double), stream));
-    if (P->chunk > 0 && c == P->chunk && !parity) {
+    if (graphs && c == P->chunk && !parity) {
       cudaGraphExec_t exec = nullptr;
       for (auto& g : P->graphs)
         if (g.chunk == c && g.blocks == blocks) exec = g.exec;
@@ -1929,7 +1944,7 @@ int run_launched(ifdtd_plan* P, const double* currents, int n, const Record* rec
         cudaError_t le = cudaSuccess;
         // an even chunk (fused plans) starts and ends in the caller's arrays
         for (int i = 0; i < c && le == cudaSuccess; ++i)
-          le = launch_step<real>(P, i, blocks, i, P->capture_stream, P->fused ? (i & 1) : 0);
+          le = launch_step<real>(P, i, {blocks, i}, P->capture_stream, P->fused ? (i & 1) : 0);
         cudaError_t ce = cudaStreamEndCapture(P->capture_stream, &graph);
         if (le != cudaSuccess) {
           if (ce == cudaSuccess) cudaGraphDestroy(graph);  // the partial capture is not kept
@@ -1942,19 +1957,18 @@ int run_launched(ifdtd_plan* P, const double* currents, int n, const Record* rec
         P->graphs.push_back({c, blocks, exec});
       }
       CUDA_TRY(cudaGraphLaunch(exec, stream));
-    } else {
-      for (int i = 0; i < c; ++i) {
-        cudaError_t e = launch_step<real>(P, i, blocks, i, stream, parity);
-        if (e != cudaSuccess) return fail(IFDTD_ERR_CUDA, std::string("step launch: ") + cudaGetErrorString(e));
-        if (P->fused) parity ^= 1;
-      }
-    }
-    if (rec)
-      for (int q = 0; q < rec->n; ++q) {
+      for (int q = 0; rec && q < rec->n; ++q) {
         const size_t r = rec->probe[q]->rows;
         CUDA_TRY(cudaMemcpyAsync(rec->out[q] + s0 * r, P->d_samples + offset[q], c * r * sizeof(double),
                                  cudaMemcpyDeviceToDevice, stream));
       }
+    } else {
+      for (int i = 0; i < c; ++i) {
+        cudaError_t e = launch_step<real>(P, i, {now_blocks, s0 + i, &now}, stream, parity);
+        if (e != cudaSuccess) return fail(IFDTD_ERR_CUDA, std::string("step launch: ") + cudaGetErrorString(e));
+        if (P->fused) parity ^= 1;
+      }
+    }
   }
   return IFDTD_OK;
 }
@@ -1999,12 +2013,10 @@ int run_steps(ifdtd_plan* P, const ifdtd_state* st, const double* currents, int 
       const int c = std::min(rec->every, n - s0);
       rc = run_launched<real>(P, currents ? currents + s0 : nullptr, c, nullptr, parity, stream);
       if (rc) break;
-      SampleSlot slots[kMaxSlots] = {};
-      for (int q = 0; q < rec->n; ++q) fill_slot(slots[q], rec->probe[q], rec->out[q]);
-      if (k == 0) CUDA_TRY(cudaMemcpyAsync(P->d_slots, slots, sizeof(slots), cudaMemcpyHostToDevice, stream));
-      sample_slots_kernel<real><<<(rec->rows() + 7) / 8, 256, 0, stream>>>(
-          (const Rec<real>*)(parity ? P->d_rec_b : P->d_rec), P->d_slots, k);
-      CUDA_TRY(cudaGetLastError());
+      SampleSlots now = {};
+      for (int q = 0; q < rec->n; ++q) fill_slot(now.slot[q], rec->probe[q], rec->out[q]);
+      CUDA_TRY(launch_after(sample_now_kernel<real>, (rec->rows() + 7) / 8, 256, 0, stream,
+                            (const Rec<real>*)(parity ? P->d_rec_b : P->d_rec), now, k));
     }
   }
   if (rc) return rc;

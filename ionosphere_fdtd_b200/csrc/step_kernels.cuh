@@ -1041,17 +1041,34 @@ __device__ __forceinline__ void sample_row(const Rec<real>& R, const SampleSlot&
   if (lane == 0) S.out[sample * S.rows + r] = acc;
 }
 
-// Every row of the slots in device memory: captured graphs name neither the
-// probes nor the fields, so one graph serves every recorded run of its plan.
+// Every row of both slots, one warp each, into row `sample` of the slots' outputs.
+template <typename real>
+__device__ __forceinline__ void sample_slots(const Rec<real>& R, const SampleSlot* slots, int sample) {
+  const int warps = gridDim.x * (blockDim.x >> 5), first = slots[0].rows, rows = first + slots[1].rows;
+  for (int w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; w < rows; w += warps)
+    sample_row(R, slots[w < first ? 0 : 1], w < first ? w : w - first, (size_t)sample);
+}
+
+// Slots in device memory, for the plan's own graphs: they name neither the probes
+// nor the fields, so one graph serves every recorded run of its plan.
 template <typename real>
 __global__ void sample_slots_kernel(const Rec<real>* __restrict__ rec, const SampleSlot* __restrict__ slots, int sample) {
   launch_next();
   wait_previous();
-  const int warps = gridDim.x * (blockDim.x >> 5);
-  for (int w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; w < slots[0].rows + slots[1].rows; w += warps) {
-    const int first = slots[0].rows;
-    sample_row(*rec, slots[w < first ? 0 : 1], w < first ? w : w - first, (size_t)sample);
-  }
+  sample_slots(*rec, slots, sample);
+}
+
+// Slots as an argument, for every other launch: nothing of the host's is read after
+// the call returns, so a capture of the caller's may be replayed for as long as the
+// probes and the outputs live.
+struct SampleSlots {
+  SampleSlot slot[kMaxSlots];
+};
+template <typename real>
+__global__ void sample_now_kernel(const Rec<real>* __restrict__ rec, const __grid_constant__ SampleSlots S, int sample) {
+  launch_next();
+  wait_previous();
+  sample_slots(*rec, S.slot, sample);
 }
 
 // One member's probe in a batched sampling launch: the member's record,
