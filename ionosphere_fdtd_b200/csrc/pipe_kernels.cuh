@@ -590,7 +590,8 @@ __device__ __forceinline__ void consumer_layers(const Rec<real>& R, unsigned cha
 
 // The phases follow one another with programmatic dependence (launch.cuh): while the
 // launch before drains, a CTA sets up its record, barriers, layer rows and lane maps,
-// none of which a step writes, and it waits before its first copy or store.  What lay
+// which the plan alone writes, by copies; it waits before its first copy or store and
+// before it reads the source current, which may be the caller's own array.  What lay
 // between two launches was 1-2 us: a step at s6 / 50 cells 84.0 -> 81.2 us, s7 / 40
 // 225.3 -> 222.3, s6 / 40 without plasma 31.6 -> 30.1, float64 s5 / 40 35.0 -> 33.2.
 template <typename real, bool PLASMA, int COPY>
@@ -643,9 +644,9 @@ __global__ void __maxnreg__(REGS) ke_tma(const Rec<real>* __restrict__ recs, int
     const int ct = threadIdx.x - 32 * W, nct = blockDim.x - 32 * W;
     Layers<real> Ls;
     consumer_layers(R, dyn_smem, Ls, ct, nct);
-    const real current = (R.n_src_er + R.n_src_et) > 0 ? (real)R.cur[istep] : real(0);
     const ELanes<real> lanes = e_lanes<real, MAXDEG, REGS>(R, Ls, ct, nct, layout);
     wait_previous();
+    const real current = (R.n_src_er + R.n_src_et) > 0 ? (real)R.cur[istep] : real(0);
     consume_ring(G, p0, p1, [&](unsigned char* st, int s, uint32_t ph) {
       ke_consume<real, PLASMA, MAXDEG, REGS>(R, Ls, lanes, st, ct, current);
     });

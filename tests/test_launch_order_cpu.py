@@ -2,7 +2,8 @@
 
 A kernel that lets its successor begin before it holds its tensor memory can wait
 for good: the successor may take the columns and then waits for the kernel's end.
-Neither wait has a bound, so the order is checked here, where nothing runs.
+Neither wait has a bound, so the order is checked here, where nothing runs.  And what
+a caller's kernel may have written just before a step is read after the wait.
 """
 
 import re
@@ -36,3 +37,11 @@ def test_tensor_memory_is_held_before_the_next_launch_begins():
     for name, body in both.items():
         held = body.index("__syncthreads()", body.index("tcgen05.alloc"))
         assert body.index("launch_next()") > held, name
+
+
+def test_source_currents_are_read_after_the_wait():
+    both = {n: b for n, b in kernels().items() if "R.cur[" in b and "wait_previous()" in b}
+    assert {"ke_tma", "ke_tma_batch"} <= both.keys()
+    for name, body in both.items():
+        assert body.rindex("wait_previous()", 0, body.index("R.cur[")) > 0, name
+        assert "wait_previous()" not in body[body.index("R.cur["):], name
