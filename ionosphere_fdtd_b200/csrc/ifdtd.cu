@@ -2168,10 +2168,8 @@ template <typename real, bool PL, int MD>
 auto batch_ke_kernel_t(const BatchGroup& g) {
   using namespace pipe;
   const int threads = g.e_threads + 32 * g.e_producers;
-  // with plasma the batched kernel spills at 128 registers and fits 96, where it re-reads its layer factors
-  constexpr int kMid = PL ? kWideRegs : kMidRegs;
   return threads > kMidMaxThreads ? ke_tma_batch<real, PL, MD, 0, kWideRegs>
-         : threads > kMaxThreads  ? ke_tma_batch<real, PL, MD, 0, kMid>
+         : threads > kMaxThreads  ? ke_tma_batch<real, PL, MD, 0, kMidRegs>
          : g.copy                 ? ke_tma_batch<real, PL, MD, 1, kMaxRegs>
                                   : ke_tma_batch<real, PL, MD, 0, kMaxRegs>;
 }
@@ -2228,8 +2226,9 @@ int batch_build(ifdtd_batch* B) {
       key.lanes = P->lanes;
       key.e_threads = P->e_threads;
       key.e_producers = P->e_producers;
-      // the batched E kernel with plasma spills at 128 registers: 8 consumer warps where the count is
-      // automatic (rows then have at most 256 quads), the count asked for otherwise
+      // the batched E kernel with plasma spills about 100 bytes at 128 registers (and at 96): 8 consumer
+      // warps at 168 where the count is automatic (a step of four s6 / 40 members 234 us, 249 with 12
+      // warps), the count asked for otherwise
       if (P->plasma && P->e_threads_auto && key.e_threads + 32 * key.e_producers == pipe::kMidMaxThreads)
         key.e_threads = pipe::kMaxThreads - 32 * key.e_producers;
     }
