@@ -77,8 +77,8 @@ typedef struct ifdtd_nn_layer {
 /* The forward pass of a network of at most 32 layers, one launch per layer: for every rows_per_pass
  * rows (a divisor of rows) the same results as ifdtd_nn_gemm_tc_ws (with 16 MiB of workspace) and
  * ifdtd_nn_bias_act layer by layer on those rows.  z may be NULL but in the last layer (a pass without
- * backward).  fan_in must be a multiple of 8 and the arrays 16-byte aligned (IFDTD_ERR_UNSUPPORTED
- * otherwise). */
+ * backward).  fan_in must be a multiple of 8, the arrays 16-byte aligned and every layer's input and
+ * output below 2^31 values (IFDTD_ERR_UNSUPPORTED otherwise). */
 int32_t ifdtd_nn_forward(const ifdtd_nn_layer* layers, int32_t n, int32_t rows, int32_t rows_per_pass, const void* x,
                          void* stream);
 /* Gradients of every weight and bias from grad = dLoss/dz of the last layer's activation, after

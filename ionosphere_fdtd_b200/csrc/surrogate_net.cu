@@ -602,7 +602,9 @@ int check_layers(const ifdtd_nn_layer* layers, int n, int rows, const void* x) {
       return record_error(IFDTD_ERR_ARGUMENT, "bad network layer");
     if (l.fan_in % 8 || !aligned16(l.w16) || !aligned16(l.z) || (l.y && !aligned16(l.y)))
       return record_error(IFDTD_ERR_UNSUPPORTED, "network layer needs fan_in in eights and 16-byte aligned arrays");
-    if (r * std::max(l.fan_out, l.fan_in) >= (int64_t)1 << 31) return record_error(IFDTD_ERR_ARGUMENT, "network layer too large");
+    // the epilogue's rows and columns are 32-bit; the separate kernels take larger layers
+    if (r * std::max(l.fan_out, l.fan_in) >= (int64_t)1 << 31)
+      return record_error(IFDTD_ERR_UNSUPPORTED, "network layer of 2^31 values or more");
     r *= l.expand;
   }
   return IFDTD_OK;

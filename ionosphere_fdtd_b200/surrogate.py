@@ -169,10 +169,16 @@ class TraceSurrogate:
 
     def _whole_pass(self, x16) -> bool:
         """Whether the one-launch-per-layer passes take this network and input: TMA
-        reads rows of whole 16-byte units."""
+        reads rows of whole 16-byte units, and a layer has less than 2^31 values."""
 
-        return (self.gemm_entry != "ifdtd_nn_gemm" and 0 < len(self.layers) <= N.NET_MAX_LAYERS and int(x16.shape[0]) > 0
-                and all(L.fan_in % 8 == 0 for L in self.layers) and x16.data_ptr() % 16 == 0)
+        rows = int(x16.shape[0])
+        if self.gemm_entry == "ifdtd_nn_gemm" or not 0 < len(self.layers) <= N.NET_MAX_LAYERS or rows <= 0 or x16.data_ptr() % 16:
+            return False
+        for L in self.layers:
+            if L.fan_in % 8 or rows * max(L.fan_in, L.fan_out) >= 1 << 31:
+                return False
+            rows *= L.expand
+        return True
 
     def _bind_weights(self):
         for d, L, w, b in zip(self._net, self.layers, self.w16, self.b):

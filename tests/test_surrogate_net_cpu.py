@@ -1,0 +1,42 @@
+"""What the surrogate's whole passes refuse before any device work, and what they
+leave to the layer-by-layer passes (no device: the addresses are never used)."""
+
+import ctypes as C
+from types import SimpleNamespace
+
+import pytest
+
+from ionosphere_fdtd_b200 import _native as N
+from ionosphere_fdtd_b200.surrogate import Layer, TraceSurrogate, architecture
+
+BASE = 1 << 40
+
+
+def _layers(shapes):
+    """Descriptors whose arrays lie at made-up 256-byte aligned addresses."""
+
+    net = (N.NetLayer * len(shapes))()
+    at = BASE
+    for d, (fan_in, fan_out, act, expand) in zip(net, shapes):
+        d.fan_in, d.fan_out, d.act, d.expand = fan_in, fan_out, act, expand
+        for name in ("w16", "bias", "z", "y", "dz", "dz16", "gw", "gb"):
+            setattr(d, name, at)
+            at += 1 << 36
+    return net
+
+
+SHAPES = [(8, 64, 1, 4), (16, 4, 0, 1)]
+
+
+@pytest.mark.parametrize("rows", [1 << 25, 1 << 26])
+def test_layers_of_2_to_the_31_values_are_left_to_the_separate_kernels(rows):
+    assert N.load().ifdtd_nn_forward(_layers(SHAPES), 2, rows, rows, BASE, None) == N.ERR_UNSUPPORTED
+    net = object.__new__(TraceSurrogate)
+    net.gemm_entry, net.layers = "ifdtd_nn_gemm_tc_ws", [Layer(*s) for s in SHAPES]
+    x = SimpleNamespace(shape=(rows, 8), data_ptr=lambda: BASE)
+    assert not net._whole_pass(x)
+    x.shape = ((1 << 25) - 1, 8)
+    assert net._whole_pass(x)
+    net.layers = architecture()
+    x.shape = (524_288, 8)
+    assert not net._whole_pass(x)
