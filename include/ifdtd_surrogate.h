@@ -85,7 +85,8 @@ int32_t ifdtd_nn_forward(const ifdtd_nn_layer* layers, int32_t n, int32_t rows, 
  * ifdtd_nn_forward on the same arrays: one launch per layer and one that finishes all layers; the same
  * results as ifdtd_nn_act_grad, ifdtd_nn_gemm_tc_ws and ifdtd_nn_col_sum layer by layer.  tickets:
  * IFDTD_NN_TICKETS zeroed int32 that every call leaves zeroed; workspace: at least
- * ifdtd_nn_backward_bytes, 16-byte aligned.  Calls that share either must not overlap on the GPU. */
+ * ifdtd_nn_backward_bytes, 16-byte aligned.  grad, dz, dz16 and gw must be 16-byte aligned too
+ * (IFDTD_ERR_UNSUPPORTED otherwise).  Calls that share either must not overlap on the GPU. */
 int32_t ifdtd_nn_backward_bytes(const ifdtd_nn_layer* layers, int32_t n, int32_t rows, int64_t* bytes);
 int32_t ifdtd_nn_backward(const ifdtd_nn_layer* layers, int32_t n, int32_t rows, const void* x, const float* grad,
                           int32_t* tickets, void* workspace, int64_t workspace_bytes, void* stream);

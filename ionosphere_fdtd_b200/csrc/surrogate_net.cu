@@ -675,14 +675,18 @@ int32_t ifdtd_nn_backward(const ifdtd_nn_layer* layers, int32_t n, int32_t rows,
   int64_t need = 0;
   rc = ifdtd_nn_backward_bytes(layers, n, rows, &need);
   if (rc) return rc;
-  if (!grad || !tickets || !workspace || !aligned16(workspace) || !aligned16(grad) || workspace_bytes < need)
+  if (!grad || !tickets || !workspace || !aligned16(workspace) || workspace_bytes < need)
     return ifdtd::record_error(IFDTD_ERR_ARGUMENT, "bad backward arguments");
+  if (!aligned16(grad)) return ifdtd::record_error(IFDTD_ERR_UNSUPPORTED, "gradient is not 16-byte aligned");
   int row_of[kMaxJobs];
   int tickets_at[kMaxJobs], n_tickets = 0;
   for (int i = 0, r = rows; i < n; ++i) {
     const ifdtd_nn_layer& l = layers[i];
-    if (!l.z || !l.gw || !l.gb || !l.dz16 || !aligned16(l.dz16) || (!l.dz && (i + 1 < n || l.act)))
+    if (!l.z || !l.gw || !l.gb || !l.dz16 || (!l.dz && (i + 1 < n || l.act)))
       return ifdtd::record_error(IFDTD_ERR_ARGUMENT, "bad network gradient arrays");
+    // the epilogues store gw, dz and dz16, and the bias sums read dz, 16 bytes at a time (gb by single values)
+    if (!aligned16(l.dz16) || !aligned16(l.dz) || !aligned16(l.gw))
+      return ifdtd::record_error(IFDTD_ERR_UNSUPPORTED, "network gradient arrays are not 16-byte aligned");
     row_of[i] = r;
     r *= l.expand;
     tickets_at[i] = n_tickets;

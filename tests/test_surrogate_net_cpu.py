@@ -40,3 +40,22 @@ def test_layers_of_2_to_the_31_values_are_left_to_the_separate_kernels(rows):
     net.layers = architecture()
     x.shape = (524_288, 8)
     assert not net._whole_pass(x)
+
+
+@pytest.mark.parametrize("name", ["gw", "dz", "dz16", "z", "y", "w16"])
+def test_unaligned_arrays_are_refused_before_a_launch(name):
+    lib, rows, need = N.load(), 300, C.c_int64()
+    net = _layers(SHAPES)
+    assert lib.ifdtd_nn_backward_bytes(net, 2, rows, C.byref(need)) == N.OK
+    setattr(net[0], name, getattr(net[0], name) + 4)
+    args = (BASE, BASE, BASE, BASE, need.value, None)
+    assert lib.ifdtd_nn_backward(net, 2, rows, *args) == N.ERR_UNSUPPORTED
+    if name in ("z", "y", "w16"):
+        assert lib.ifdtd_nn_forward(net, 2, rows, rows, BASE, None) == N.ERR_UNSUPPORTED
+
+
+def test_an_unaligned_gradient_is_refused_before_a_launch():
+    lib, rows, need = N.load(), 300, C.c_int64()
+    net = _layers(SHAPES)
+    assert lib.ifdtd_nn_backward_bytes(net, 2, rows, C.byref(need)) == N.OK
+    assert lib.ifdtd_nn_backward(net, 2, rows, BASE, BASE + 4, BASE, BASE, need.value, None) == N.ERR_UNSUPPORTED
