@@ -24,6 +24,7 @@ HEADERS = [
     PACKAGE / "csrc" / "loop_kernels.cuh",
     PACKAGE / "csrc" / "errors.cuh",
     PACKAGE / "csrc" / "launch.cuh",
+    PACKAGE / "csrc" / "raise_limit.h",
     PACKAGE / "csrc" / "silu.cuh",
     PACKAGE / "csrc" / "tc_common.cuh",
     ROOT / "include" / "ifdtd.h",

@@ -18,6 +18,7 @@
 #include "fused_kernels.cuh"
 #include "loop_kernels.cuh"
 #include "pipe_kernels.cuh"
+#include "raise_limit.h"
 #include "step_kernels.cuh"
 
 using namespace ifdtd;
@@ -1698,11 +1699,15 @@ int bind_state(ifdtd_plan* P, const ifdtd_state* st, cudaStream_t stream) {
 template <typename K>
 cudaError_t allow_smem(K kernel, size_t bytes) {
   if (bytes <= 48 * 1024) return cudaSuccess;
-  cudaFuncAttributes attr;
-  cudaError_t e = cudaFuncGetAttributes(&attr, kernel);
-  if (e != cudaSuccess) return e;
-  if ((size_t)attr.maxDynamicSharedSizeBytes >= bytes) return cudaSuccess;
-  return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+  return raise_limit(
+      bytes,
+      [&](size_t* now) {
+        cudaFuncAttributes attr;
+        const cudaError_t e = cudaFuncGetAttributes(&attr, kernel);
+        if (e == cudaSuccess) *now = (size_t)attr.maxDynamicSharedSizeBytes;
+        return e;
+      },
+      [&](size_t b) { return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)b); });
 }
 
 // allow_smem once per plan and launch kind (the query costs more than a launch).
