@@ -101,7 +101,6 @@ class TraceSurrogate:
                 lst.append(torch.zeros(shape, dtype=torch.float32, device=self.device))
         self.step_count = 0
         self._acts: list = []
-        self._net = (N.NetLayer * len(layers))()
         self._layout: tuple | None = None  # of the last batch size
 
     # -- the last pass: activations (input, pre-activation per layer) and gradients.
@@ -181,10 +180,13 @@ class TraceSurrogate:
         return True
 
     def _bind_weights(self):
-        for d, L, w, b in zip(self._net, self.layers, self.w16, self.b):
+        """The layers' descriptors, this call's own: another thread may be in a pass of this model."""
+
+        net = (N.NetLayer * len(self.layers))()
+        for d, L, w, b in zip(net, self.layers, self.w16, self.b):
             d.fan_in, d.fan_out, d.act, d.expand = L.fan_in, L.fan_out, L.act, L.expand
             d.w16, d.bias = w.data_ptr(), b.data_ptr()
-        return self._net
+        return net
 
     @staticmethod
     def _offsets(sizes) -> tuple[list[int], int]:
@@ -199,7 +201,8 @@ class TraceSurrogate:
     def _batch_layout(self, batch: int) -> tuple:
         """(batch, rows of every layer, outputs per case, forward offsets and bytes, backward scratch offsets and bytes)."""
 
-        if self._layout is None or self._layout[0] != batch:
+        layout = self._layout
+        if layout is None or layout[0] != batch:
             rows = [batch]
             for L in self.layers[:-1]:
                 rows.append(rows[-1] * L.expand)
@@ -209,8 +212,8 @@ class TraceSurrogate:
             work = int(need.value)
             scratch = self._offsets([4 * r * L.fan_out for r, L in zip(rows, self.layers)]
                                     + [2 * r * ((L.fan_out + 7) // 8 * 8) for r, L in zip(rows, self.layers)] + [work])
-            self._layout = (batch, rows, rows[-1] * self.layers[-1].fan_out // batch, forward, scratch, work)
-        return self._layout
+            layout = self._layout = (batch, rows, rows[-1] * self.layers[-1].fan_out // batch, forward, scratch, work)
+        return layout
 
     def _block(self, size: int):
         return self.torch.empty(size, dtype=self.torch.uint8, device=self.device)

@@ -2,11 +2,13 @@
 leave to the layer-by-layer passes (no device: the addresses are never used)."""
 
 import ctypes as C
+import threading
 from types import SimpleNamespace
 
 import pytest
 
 from ionosphere_fdtd_b200 import _native as N
+from ionosphere_fdtd_b200 import surrogate
 from ionosphere_fdtd_b200.surrogate import Layer, TraceSurrogate, architecture
 
 BASE = 1 << 40
@@ -59,3 +61,36 @@ def test_an_unaligned_gradient_is_refused_before_a_launch():
     net = _layers(SHAPES)
     assert lib.ifdtd_nn_backward_bytes(net, 2, rows, C.byref(need)) == N.OK
     assert lib.ifdtd_nn_backward(net, 2, rows, BASE, BASE + 4, BASE, BASE, need.value, None) == N.ERR_UNSUPPORTED
+
+
+@pytest.mark.parametrize("infer", [False, True])
+def test_passes_of_two_threads_keep_their_own_arrays(monkeypatch, infer):
+    """Both threads have described their pass before either is enqueued."""
+
+    import torch
+
+    met, enqueued = threading.Barrier(2, timeout=30), {}
+
+    def forward(net, n, rows, rows_per_pass, x, stream):
+        met.wait()
+        enqueued[x] = (rows, net[n - 1].z)
+        return N.OK
+
+    monkeypatch.setattr(surrogate, "_lib", lambda: SimpleNamespace(
+        ifdtd_nn_forward=forward, ifdtd_nn_backward_bytes=N.load().ifdtd_nn_backward_bytes))
+    model = object.__new__(TraceSurrogate)
+    model.torch, model.device, model.gemm_entry = torch, torch.device("cpu"), "ifdtd_nn_gemm_tc_ws"
+    model.layers = [Layer(*s) for s in SHAPES]
+    model._layout = None
+    model.w16 = [torch.zeros((L.fan_out, L.fan_in), dtype=torch.bfloat16) for L in model.layers]
+    model.b = [torch.zeros(L.fan_out) for L in model.layers]
+    monkeypatch.setattr(TraceSurrogate, "_stream", lambda self: None)
+    xs = [torch.zeros((rows, 8), dtype=torch.bfloat16) for rows in (24, 40)]
+    outs = [torch.zeros((len(x), 16)) for x in xs]
+    run = (lambda x, o: model._infer(x, len(x), o)) if infer else model._forward
+    threads = [threading.Thread(target=run, args=a) for a in zip(xs, outs)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert enqueued == {x.data_ptr(): (len(x), o.data_ptr()) for x, o in zip(xs, outs)}
