@@ -418,7 +418,7 @@ class TraceSurrogate:
             samples *= L.expand
         out = torch.empty((rows, samples), dtype=torch.float32, device=self.device)
         # the batches but the last in groups of several per pass, the last as a plain
-        # forward pass (its activations stay for a backward pass)
+        # forward pass (its activations stay for a backward pass, so its rows are copied)
         group = batch * max(1, GROUP_ROWS // batch)
         i, last = 0, (rows - 1) // batch * batch
         while i < last:
@@ -427,7 +427,7 @@ class TraceSurrogate:
                 n = batch
                 self._forward(x[i : i + n].contiguous(), out[i : i + n])
             i += n
-        self._forward(x[last:].contiguous(), out[last:])
+        out[last:].copy_(self._forward(x[last:].contiguous(), None))
         return out
 
 

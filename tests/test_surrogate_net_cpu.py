@@ -63,6 +63,22 @@ def test_an_unaligned_gradient_is_refused_before_a_launch():
     assert lib.ifdtd_nn_backward(net, 2, rows, BASE, BASE + 4, BASE, BASE, need.value, None) == N.ERR_UNSUPPORTED
 
 
+def _hostless(monkeypatch, forward, shapes):
+    """A model on host tensors whose forward launches are ``forward``."""
+
+    import torch
+
+    monkeypatch.setattr(surrogate, "_lib", lambda: SimpleNamespace(
+        ifdtd_nn_forward=forward, ifdtd_nn_backward_bytes=N.load().ifdtd_nn_backward_bytes))
+    monkeypatch.setattr(TraceSurrogate, "_stream", lambda self: None)
+    model = object.__new__(TraceSurrogate)
+    model.torch, model.device, model.gemm_entry = torch, torch.device("cpu"), "ifdtd_nn_gemm_tc_ws"
+    model.layers, model._layout = [Layer(*s) for s in shapes], None
+    model.w16 = [torch.zeros((L.fan_out, L.fan_in), dtype=torch.bfloat16) for L in model.layers]
+    model.b = [torch.zeros(L.fan_out) for L in model.layers]
+    return model
+
+
 @pytest.mark.parametrize("infer", [False, True])
 def test_passes_of_two_threads_keep_their_own_arrays(monkeypatch, infer):
     """Both threads have described their pass before either is enqueued."""
@@ -76,15 +92,7 @@ def test_passes_of_two_threads_keep_their_own_arrays(monkeypatch, infer):
         enqueued[x] = (rows, net[n - 1].z)
         return N.OK
 
-    monkeypatch.setattr(surrogate, "_lib", lambda: SimpleNamespace(
-        ifdtd_nn_forward=forward, ifdtd_nn_backward_bytes=N.load().ifdtd_nn_backward_bytes))
-    model = object.__new__(TraceSurrogate)
-    model.torch, model.device, model.gemm_entry = torch, torch.device("cpu"), "ifdtd_nn_gemm_tc_ws"
-    model.layers = [Layer(*s) for s in SHAPES]
-    model._layout = None
-    model.w16 = [torch.zeros((L.fan_out, L.fan_in), dtype=torch.bfloat16) for L in model.layers]
-    model.b = [torch.zeros(L.fan_out) for L in model.layers]
-    monkeypatch.setattr(TraceSurrogate, "_stream", lambda self: None)
+    model = _hostless(monkeypatch, forward, SHAPES)
     xs = [torch.zeros((rows, 8), dtype=torch.bfloat16) for rows in (24, 40)]
     outs = [torch.zeros((len(x), 16)) for x in xs]
     run = (lambda x, o: model._infer(x, len(x), o)) if infer else model._forward
@@ -94,3 +102,20 @@ def test_passes_of_two_threads_keep_their_own_arrays(monkeypatch, infer):
     for t in threads:
         t.join()
     assert enqueued == {x.data_ptr(): (len(x), o.data_ptr()) for x, o in zip(xs, outs)}
+
+
+@pytest.mark.parametrize("cases", [16, 40, 100])
+def test_a_prediction_is_not_the_kept_activations(monkeypatch, cases):
+    """A program may overwrite its predictions before it asks for gradients."""
+
+    import torch
+
+    def forward(net, n, rows, rows_per_pass, x, stream):
+        C.memset(net[n - 1].z, 0, rows * 16 * 4)
+        return N.OK
+
+    model = _hostless(monkeypatch, forward, SHAPES)
+    out = model.predict(torch.zeros((cases, 8), dtype=torch.bfloat16), batch=16)
+    assert out.shape == (cases, 16) and not out.any()
+    out.fill_(7.0)
+    assert not model._acts[-1][1].any()
