@@ -68,7 +68,8 @@ def architecture(inputs: int = 8, width: int = 512, depth: int = 4, samples: int
 
 
 GEMM_ENTRIES = {"tcgen05": "ifdtd_nn_gemm_tc_ws", "mma": "ifdtd_nn_gemm"}
-GROUP_ROWS = 4096  # cases per pass of a prediction (about 100 MB of bf16 activations)
+GROUP_ROWS = 4096  # cases per pass of a prediction (about 80 MB of bf16 activations in the default network) and
+GROUP_BYTES = 256 << 20  # the activations' most, unless one batch takes more: the caller's batch bounds the memory
 WORKSPACE_BYTES = 16 << 20  # split-K partial tiles of the tcgen05 GEMM
 
 
@@ -413,13 +414,15 @@ class TraceSurrogate:
         torch, rows = self.torch, int(x.shape[0])
         if not range(0, rows, batch):
             return torch.cat([])  # refused by torch: there is nothing to predict
-        samples = self.layers[-1].fan_out
+        samples, kept = 1, 0  # outputs, and activation bytes, per case
         for L in self.layers[:-1]:
+            kept += 2 * samples * L.fan_out
             samples *= L.expand
+        samples *= self.layers[-1].fan_out
         out = torch.empty((rows, samples), dtype=torch.float32, device=self.device)
         # the batches but the last in groups of several per pass, the last as a plain
         # forward pass (its activations stay for a backward pass, so its rows are copied)
-        group = batch * max(1, GROUP_ROWS // batch)
+        group = batch * max(1, min(GROUP_ROWS, GROUP_BYTES // max(kept, 1)) // batch)
         i, last = 0, (rows - 1) // batch * batch
         while i < last:
             n = min(group, last - i)

@@ -119,3 +119,25 @@ def test_a_prediction_is_not_the_kept_activations(monkeypatch, cases):
     assert out.shape == (cases, 16) and not out.any()
     out.fill_(7.0)
     assert not model._acts[-1][1].any()
+
+
+def test_grouped_batches_are_bounded_in_memory(monkeypatch):
+    """The caller's batch bounds a prediction's memory: several batches share a pass
+    only while their activations stay small."""
+
+    import torch
+
+    rows = []
+
+    def forward(net, n, count, rows_per_pass, x, stream):
+        rows.append(count)
+        return N.OK
+
+    wide = 1 << 20  # 2 MiB of activations per case
+    model = _hostless(monkeypatch, forward, [(8, wide, 1, wide // 8), (8, 1, 0, 1)])
+    model.predict(torch.zeros((300, 8), dtype=torch.bfloat16), batch=8)
+    assert sum(rows) == 300 and rows[-1] == 4
+    assert max(rows) * 2 * wide <= 256 << 20
+    rows.clear()
+    model.predict(torch.zeros((300, 8), dtype=torch.bfloat16), batch=150)
+    assert rows == [150, 150]
