@@ -1789,6 +1789,12 @@ cudaError_t launch_ke(ifdtd_plan* P, int istep, cudaStream_t st) {
 // Up to kLoopSteps leapfrog steps in one cooperative launch, one CTA per SM (a
 // bound on one launch's time, 1-7 ms; more steps per launch gain nothing).
 constexpr int kLoopSteps = 256;
+// Most receiver rows of a loop launch per SM, whose one sampling warp takes them one
+// after the other (0.65 us each beyond what a phase hides); more are recorded on ring
+// launches.  us a step with 600, 1,200 and 2,500 rows, loop against ring: s5 / 24 cells
+// 12.2 / 14.9, 14.9 / 15.1, 20.6 / 15.3; s5 / 37 14.6 / 17.1, 17.0 / 17.1, 22.6 / 17.3;
+// s4 / 31 with 600 and 2,562 9.2 / 11.9, 18.6 / 12.5.
+constexpr int kLoopRows = 8;
 template <typename real, bool PL, int MD>
 cudaError_t launch_loop_t(ifdtd_plan* P, const LoopArgs& args, cudaStream_t st) {
   auto k = kd_loop<real, PL, MD>;
@@ -1909,10 +1915,11 @@ int run_launched(ifdtd_plan* P, const double* currents, int n, const Record* rec
   // capture never holds them (it refuses graph launches), only launches that carry their
   // slots and write the caller's rows.
   const bool graphs = P->chunk > 0 && n >= cap;
-  // blocks of a sampling launch (8 rows each); in a graph powers of two, so a plan keeps few graphs
+  // Blocks of a sampling launch: a warp per row (8 rows a block), since a row is two
+  // dependent trips to L2; in a graph the next power of two, so a plan keeps few graphs.
   const int rows = rec ? rec->rows() : 0, now_blocks = (rows + 7) / 8;
   int blocks = rec ? 1 : 0;
-  while (blocks && blocks < 64 && 8 * blocks < rows) blocks *= 2;
+  while (blocks && blocks < now_blocks) blocks *= 2;
   SampleSlots now = {};
   for (int q = 0; rec && q < rec->n; ++q) fill_slot(now.slot[q], rec->probe[q], rec->out[q]);
   size_t offset[kMaxSlots] = {0, 0};
@@ -2008,7 +2015,7 @@ int run_steps(ifdtd_plan* P, const ifdtd_state* st, const double* currents, int 
     ~Range() { nvtxRangePop(); }
   } range(rec ? "ifdtd_step_sampled" : "ifdtd_step");
   int parity = 0;
-  if (P->loop) {
+  if (P->loop && (!rec || rec->rows() <= kLoopRows * P->sm_count)) {
     rc = run_looped<real>(P, currents, n, rec, stream);
   } else if (!rec || rec->every == 1) {
     rc = run_launched<real>(P, currents, n, rec, parity, stream);
