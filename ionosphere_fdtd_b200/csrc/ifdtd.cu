@@ -298,31 +298,37 @@ bool build_pipe_h(PipeTables& T, int n, int fpp, int nF, const std::vector<int>&
   const int rb = (int)sizeof(real);
   if (Tsi > 0 && (Tsi * rb) % 16 != 0) return false;  // pole rows must be whole 16-byte units
   std::vector<real> sis;
-  std::vector<int> er_ids, et_ids;
+  std::vector<int> er_ids, et_ids, halo, seen_v(locA.size(), -1), seen_e(locB.size(), -1);
   std::vector<std::pair<int, int>> er_runs, et_runs;
   std::vector<int4> eloc, floc;
   for (int q = 0; q < n; ++q) {
     const int fa = q * fpp, fb = std::min(fa + fpp, nF), ea = eptr[q], eb = eptr[q + 1], ne = eb - ea, nf = fb - fa;
+    // each row once, then sorted: the owned edges are a run among the face edges, so only the halo needs it
     er_ids.clear();
     et_ids.clear();
-    for (int e = ea; e < eb; ++e) {
-      er_ids.push_back(th[e].x);
-      er_ids.push_back(th[e].y);
-    }
+    halo.clear();
+    int n_own = 0;
+    auto vertex = [&](int v) {
+      if (seen_v[v] != q) seen_v[v] = q, er_ids.push_back(v);
+    };
+    auto edge = [&](int e) {
+      if (seen_e[e] == q) return;
+      seen_e[e] = q;
+      if (e >= ea && e < eb) ++n_own;
+      else halo.push_back(e);
+    };
+    for (int e = ea; e < eb; ++e) vertex(th[e].x), vertex(th[e].y);
     for (int f = fa; f < fb; ++f) {
-      et_ids.push_back(fe[f].x);
-      et_ids.push_back(fe[f].y);
-      et_ids.push_back(fe[f].z);
-      if (S > 0) {
-        er_ids.push_back(fv[f].x);
-        er_ids.push_back(fv[f].y);
-        er_ids.push_back(fv[f].z);
-      }
+      edge(fe[f].x), edge(fe[f].y), edge(fe[f].z);
+      if (S > 0) vertex(fv[f].x), vertex(fv[f].y), vertex(fv[f].z);
     }
-    sort_unique(er_ids);
-    sort_unique(et_ids);
-    for (int e = ea; e < eb; ++e)
-      if (!std::binary_search(et_ids.begin(), et_ids.end(), e)) return false;
+    if (n_own != ne) return false;  // an owned edge beside none of the owned faces
+    std::sort(er_ids.begin(), er_ids.end());
+    std::sort(halo.begin(), halo.end());
+    const auto above = std::lower_bound(halo.begin(), halo.end(), ea);
+    et_ids.assign(halo.begin(), above);
+    for (int e = ea; e < eb; ++e) et_ids.push_back(e);
+    et_ids.insert(et_ids.end(), above, halo.end());
     int gap = 0, n_er = 0, n_et = 0, nd = 0;
     for (;;) {
       n_er = make_runs(er_ids, gap, er_runs, locA);
