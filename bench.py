@@ -125,6 +125,16 @@ def kernel_bytes(sim) -> dict[str, int]:
     return {"h_phase": item * (e + 2 * (h + j + si)), "e_phase": item * (h + j + 2 * e)}
 
 
+def step_launches(steps: int, rows: int, loop: tuple[int, int], fused: bool = False) -> int:
+    """Launches of a recorded run of ``steps`` steps and ``rows`` receivers: one per whole or
+    started ``loop[0]`` steps where the plan's loop kernel takes the run (``Engine.loop_launch``),
+    else the H phase, the E phase (one launch for both in a fused plan) and the sampling of
+    every step."""
+
+    per_launch, most_rows = loop
+    return -(-steps // per_launch) if per_launch and rows <= most_rows else (2 if fused else 3) * steps
+
+
 def phase_times_ms(sim, reps: int) -> dict[str, float]:
     """Median device time of each phase kernel: CUDA events around every launch on the
     launching stream (``ifdtd_time_phases``, the plasma current turned into the plan's
@@ -968,6 +978,7 @@ def main() -> None:
     }
     config = workload_config(args.workload, args.subdivision, world)
     n_species, face_frames = eng.species, eng.face_frames
+    run_launches = step_launches(T, v.shape[0], eng.loop_launch, modes[0] == "fused")
     del wl, sim, eng
     torch.cuda.empty_cache()
     drift = None
@@ -1009,15 +1020,18 @@ def main() -> None:
             "autotune": tuning,
             "hbm_gbs": achieved,
             "kernel_modes": list(modes),
+            # the kernels of the timed region; the per-kernel roofline above times the phases' own launches
+            "step_kernels": (["kd_loop"] if run_launches < T else ["kf_tma" if modes[1] == "pipeline" else "fused_step_kernel"]
+                             if modes[0] == "fused" else [names["h_phase"], names["e_phase"]]),
             "plasma_frame": {0: "auto: face frames (unmagnetised plasma)", 1: "cartesian", 2: "face frames"}[args.plasma_frame],
             "roofline": roofline,
             "cpu_baseline": cpu,
             "e2e": e2e,
             "fp32_drift": drift,
             "traces_finite": trace_finite,
-            # per bench step: H phase, E phase and sampling per leapfrog step, and with the plasma
-            # current in face frames one conversion per species each way around the call
-            "gpu_launches": (3 * T + (2 * n_species if face_frames else 0)) * K,
+            # per bench step: the run's launches, and with the plasma current in face frames one
+            # conversion per species each way around the call
+            "gpu_launches": (run_launches + (2 * n_species if face_frames else 0)) * K,
             "clocks": clocks,
             "ensemble": ensemble,
         }

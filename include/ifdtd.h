@@ -185,8 +185,14 @@ int32_t ifdtd_status_word(ifdtd_plan* plan, int32_t reset, int32_t* out);
 int32_t ifdtd_wait_selftest(ifdtd_plan* plan, double* waited_seconds, void* stream);
 /* Which step kernels the plan launches: 1 direct gathers, 2 shared-memory
  * pipeline (H phase, E phase); h_mode 3: the fused one-launch step, whose
- * kernel family e_mode gives. */
+ * kernel family e_mode gives.  Plans that step in the loop kernel (ifdtd_plan_loop)
+ * launch these for single phases, in a batch and in allocation-free steps. */
 int32_t ifdtd_plan_kernels(const ifdtd_plan* plan, int32_t* h_mode, int32_t* e_mode);
+/* Whether ifdtd_step and the recorded runs go through the loop kernel: steps
+ * receives the most leapfrog steps of one launch (0: a launch or more per step),
+ * rows the most receiver rows of a run recorded in it (0 likewise); a run of more
+ * rows launches its phases.  Either may be NULL. */
+int32_t ifdtd_plan_loop(const ifdtd_plan* plan, int32_t* steps, int32_t* rows);
 /* Bytes of device memory held by the plan (tables, staging, scratch). */
 int32_t ifdtd_plan_bytes(const ifdtd_plan* plan, int64_t* bytes);
 

@@ -1801,6 +1801,7 @@ constexpr int kLoopSteps = 256;
 // 12.2 / 14.9, 14.9 / 15.1, 20.6 / 15.3; s5 / 37 14.6 / 17.1, 17.0 / 17.1, 22.6 / 17.3;
 // s4 / 31 with 600 and 2,562 9.2 / 11.9, 18.6 / 12.5.
 constexpr int kLoopRows = 8;
+int loop_rows(const ifdtd_plan* P) { return kLoopRows * P->sm_count; }
 template <typename real, bool PL, int MD>
 cudaError_t launch_loop_t(ifdtd_plan* P, const LoopArgs& args, cudaStream_t st) {
   auto k = kd_loop<real, PL, MD>;
@@ -2021,7 +2022,7 @@ int run_steps(ifdtd_plan* P, const ifdtd_state* st, const double* currents, int 
     ~Range() { nvtxRangePop(); }
   } range(rec ? "ifdtd_step_sampled" : "ifdtd_step");
   int parity = 0;
-  if (P->loop && (!rec || rec->rows() <= kLoopRows * P->sm_count)) {
+  if (P->loop && (!rec || rec->rows() <= loop_rows(P))) {
     rc = run_looped<real>(P, currents, n, rec, stream);
   } else if (!rec || rec->every == 1) {
     rc = run_launched<real>(P, currents, n, rec, parity, stream);
@@ -2637,6 +2638,13 @@ int32_t ifdtd_plan_kernels(const ifdtd_plan* plan, int32_t* h_mode, int32_t* e_m
   if (!plan || !h_mode || !e_mode) return fail(IFDTD_ERR_ARGUMENT, "null argument");
   *h_mode = plan->fused ? 3 : plan->h_mode;
   *e_mode = plan->fused ? (plan->fused_pipe ? 2 : 1) : plan->e_mode;
+  return IFDTD_OK;
+}
+
+int32_t ifdtd_plan_loop(const ifdtd_plan* plan, int32_t* steps, int32_t* rows) {
+  if (!plan) return fail(IFDTD_ERR_ARGUMENT, "null argument");
+  if (steps) *steps = plan->loop ? kLoopSteps : 0;
+  if (rows) *rows = plan->loop ? loop_rows(plan) : 0;
   return IFDTD_OK;
 }
 

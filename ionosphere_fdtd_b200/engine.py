@@ -225,12 +225,23 @@ class Engine:
     def kernel_modes(self) -> tuple[str, str]:
         """Kernel family of the H and E phases: "direct" (global gathers) or
         "pipeline" (warp-specialised shared-memory pipeline); a fused plan
-        reports ("fused", family of its one-launch kernel)."""
+        reports ("fused", family of its one-launch kernel).  A plan whose runs
+        go through the loop kernel (``loop_launch``) launches these for single
+        phases and as a member of an ensemble."""
 
         h, e = C.c_int32(), C.c_int32()
         N.check(N.load().ifdtd_plan_kernels(self.plan, C.byref(h), C.byref(e)), "ifdtd_plan_kernels")
         name = {1: "direct", 2: "pipeline", 3: "fused"}
         return name[h.value], name[e.value]
+
+    @property
+    def loop_launch(self) -> tuple[int, int]:
+        """Most leapfrog steps of one launch of the loop kernel, and most receiver
+        rows of a run recorded in it; (0, 0) for a plan that launches its phases."""
+
+        steps, rows = C.c_int32(), C.c_int32()
+        N.check(N.load().ifdtd_plan_loop(self.plan, C.byref(steps), C.byref(rows)), "ifdtd_plan_loop")
+        return int(steps.value), int(rows.value)
 
     def status_word(self, reset: bool = False) -> int:
         out = C.c_int32()
