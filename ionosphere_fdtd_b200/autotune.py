@@ -10,16 +10,18 @@ restores that state, and installs the fastest plan.  Every candidate computes
 the same bits (patch size, lane layout, kernel family and the fused
 one-launch step do not change any result; every candidate keeps the
 simulation's plasma frame, which does), so tuning changes speed only.  ``autotune_ensemble`` tunes the largest member
-of each class (by default: mesh level, radial cells, precision and physics)
-and gives the winner to the whole class.
+of each class (by default: mesh level, radial cells, precision and physics),
+in batched launches, and gives the winner to the whole class.
 """
 
 from __future__ import annotations
 
+import ctypes as C
 import statistics
 from dataclasses import dataclass, field, replace
 from typing import Sequence
 
+from . import _native as N
 from .engine import Engine, Tuning
 from .errors import BackendUnavailableError
 
@@ -78,20 +80,40 @@ def _engine_for(sim, tuning: Tuning) -> Engine:
                   sim.backend, tuning)
 
 
-def _time_engine(sim, engine: Engine, steps: int, repeats: int) -> float:
+def _median_ms(sim, run, steps: int, repeats: int) -> float:
     torch = sim.backend.torch
     stream = torch.cuda.current_stream(sim.backend.torch_device)
-    state = sim._state()
-    engine.step(state, None, steps)  # warm-up: captures the step graphs
+    run()  # warm-up: captures the step graphs
     times = []
     for _ in range(repeats):
         a, b = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
         a.record(stream)
-        engine.step(state, None, steps)
+        run()
         b.record(stream)
         b.synchronize()
         times.append(a.elapsed_time(b) / steps)
     return statistics.median(times)
+
+
+def _time_engine(sim, engine: Engine, steps: int, repeats: int) -> float:
+    state = sim._state()
+    return _median_ms(sim, lambda: engine.step(state, None, steps), steps, repeats)
+
+
+def _time_in_batch(sim, engine: Engine, steps: int, repeats: int) -> float:
+    """As an ensemble runs the plan: its batched launches, never the loop kernel."""
+
+    states = (N.State * 1)(sim._state())
+    handle = C.c_void_p()
+    N.check(N.load().ifdtd_batch_create((C.c_void_p * 1)(engine.plan.value), 1, 32, C.byref(handle)), "ifdtd_batch_create")
+
+    def run():
+        N.check(N.load().ifdtd_batch_step(handle, states, None, steps, None, None, sim.backend.stream_handle()), "ifdtd_batch_step")
+
+    try:
+        return _median_ms(sim, run, steps, repeats)
+    finally:
+        N.load().ifdtd_batch_destroy(handle)
 
 
 def autotune(sim, candidates: Sequence[Tuning] = DEFAULT_CANDIDATES, *, steps: int = 32, repeats: int = 3) -> AutotuneResult:
@@ -105,6 +127,10 @@ def autotune(sim, candidates: Sequence[Tuning] = DEFAULT_CANDIDATES, *, steps: i
     stage does not fit twice in shared memory), or whose launches the device
     refuses, is recorded with its error."""
 
+    return _tune(sim, candidates, steps, repeats, _time_engine)
+
+
+def _tune(sim, candidates: Sequence[Tuning], steps: int, repeats: int, timer) -> AutotuneResult:
     if steps < 1 or repeats < 1:
         raise ValueError("steps and repeats must be positive")
     if not candidates:
@@ -124,7 +150,7 @@ def autotune(sim, candidates: Sequence[Tuning] = DEFAULT_CANDIDATES, *, steps: i
                 result.timings.append((tuning, None, str(err)))
                 continue
             try:
-                ms = _time_engine(sim, engine, steps, repeats)
+                ms = timer(sim, engine, steps, repeats)
             except RuntimeError as err:
                 # a launch the device refuses (for example a launch shape with no
                 # resident CTA) is recorded like a plan the builder rejects
@@ -183,8 +209,8 @@ SHAPE_FREE_CANDIDATES: tuple[Tuning, ...] = (
 
 def autotune_ensemble(members: Sequence, candidates: Sequence[Tuning] = DEFAULT_CANDIDATES, *, steps: int = 32,
                       repeats: int = 3, key=None) -> dict[tuple, AutotuneResult]:
-    """Tune the largest member of every class and install the winner on the
-    rest of the class.  Classes default to (subdivision, radial cells,
+    """Tune the largest member of every class, timed in the batched launches that
+    the ensemble runs, and install the winner on the rest of the class.  Classes default to (subdivision, radial cells,
     precision, plasma, surface impedance); ``key`` may map a member to a
     coarser class (then use candidates that fix no patch size, such as
     ``SHAPE_FREE_CANDIDATES``).  Call it before building the ``Ensemble``: the
@@ -197,7 +223,7 @@ def autotune_ensemble(members: Sequence, candidates: Sequence[Tuning] = DEFAULT_
         group.sort(key=lambda m: -m.mesh.n_vertices * m.config.radial_cells)
     out = {}
     for cls, group in classes.items():
-        res = autotune(group[0], candidates, steps=steps, repeats=repeats)
+        res = _tune(group[0], candidates, steps, repeats, _time_in_batch)
         out[cls] = res
         for m in group[1:]:
             if m._engine.tuning != res.best:
