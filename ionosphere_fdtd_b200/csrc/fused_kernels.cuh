@@ -54,8 +54,11 @@ __device__ __forceinline__ void st_shared16(real* p, const Run<real>& r) {
   }
 }
 
+// Bound by the gathers' latency: up to 64 registers for loads in flight and four CTAs per
+// SM.  Left to itself the compiler took 48 and five CTAs in float64, which thrash L1:
+// 118.5 us a step at s6 / 20 cells instead of 88.9, 136 instead of 101 at s6 / 24.
 template <typename real, int MAXDEG>
-__global__ void __launch_bounds__(256) fused_step_kernel(const Rec<real>* __restrict__ rin,
+__global__ void __launch_bounds__(256, 4) fused_step_kernel(const Rec<real>* __restrict__ rin,
                                                          const Rec<real>* __restrict__ rout, FusedTables ft, int istep) {
   constexpr int N = Lanes<real>::N;
   extern __shared__ __align__(16) unsigned char dyn_smem[];
