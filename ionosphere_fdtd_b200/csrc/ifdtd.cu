@@ -138,7 +138,7 @@ struct ifdtd_plan {
   void* spare = nullptr;
   size_t spare_bytes = 0;
   SampleSlot* d_slots = nullptr;  // the run's probes as the sampling launches of the plan's graphs read them
-  double* d_samples = nullptr;    // (graph_chunk, rows) of each slot
+  double* d_samples = nullptr;    // (graph_chunk, rows) of each slot; given back with a run's probes above kSpareSamples
   size_t sample_values = 0;
   unsigned opted = 0;  // launch kinds whose shared-memory limit is raised
   std::vector<float> kh_cost, ke_cost;  // staged bytes per pipelined patch (balances batched launches)
@@ -164,6 +164,7 @@ struct ifdtd_plan {
 namespace {
 
 constexpr size_t kSpareBytes = (size_t)1 << 20;
+constexpr size_t kSpareSamples = ((size_t)16 << 20) / sizeof(double);  // kept by a plan between recorded runs
 
 template <typename real>
 std::vector<real> cast(const double* p, size_t n) {
@@ -2810,6 +2811,11 @@ int32_t ifdtd_probe_destroy(ifdtd_probe* probe) {
     if (probe->bytes <= kSpareBytes && probe->bytes > plan->spare_bytes) {
       std::swap(probe->block, plan->spare);
       std::swap(probe->bytes, plan->spare_bytes);
+    }
+    if (plan->sample_values > kSpareSamples) {
+      cudaFree(plan->d_samples);
+      plan->d_samples = nullptr;
+      plan->sample_values = 0;
     }
   }
   delete probe;

@@ -84,3 +84,25 @@ def test_a_row_for_every_vertex_costs_a_sampling_launch(level, cells):
         sample = _us_per_step(samples, steps)
         probe.close()
         assert sampled < 1.5 * (step + sample), (level, sampled, step, sample)
+
+
+def test_a_plan_gives_large_sample_rows_back():
+    """32 steps of 300,000 rows are 77 MB of staging: gone with the run's probe."""
+
+    import torch
+
+    (sim,) = _sims(dict(staging=2))
+    v, k, w = _receivers(sim, 300_000)
+    first = sim.record_er_observations(v[:8], k[:8, 0], w[:8], 40)
+    before = torch.cuda.mem_get_info()[0]
+    probe = sim._engine.probe("er", v, k, w)
+    out = torch.zeros((32, len(v)), dtype=torch.float64, device="cuda")
+    taken = torch.cuda.mem_get_info()[0]
+    sim._engine.step_sampled(sim._state(), None, 32, probe, out)
+    torch.cuda.synchronize()
+    assert taken - torch.cuda.mem_get_info()[0] > 60e6
+    probe.close()
+    held = out.numel() * 8 + 4e6
+    assert before - torch.cuda.mem_get_info()[0] < held + 20e6
+    again = sim.record_er_observations(v[:8], k[:8, 0], w[:8], 40)  # the plan's graphs, on new staging
+    assert np.isfinite(first).all() and np.abs(again).max() > 0.0
