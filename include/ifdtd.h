@@ -254,7 +254,10 @@ int32_t ifdtd_probe_destroy(ifdtd_probe* probe);
 int32_t ifdtd_sample(ifdtd_plan* plan, const ifdtd_state* state, const ifdtd_probe* probe,
                      double* out_row, void* stream);
 /* Step n_steps times, sampling after every step into out_rows (n_steps, rows)
- * (record_er_observations' inner loop, solver.py:1126-1135). */
+ * (record_er_observations' inner loop, solver.py:1126-1135).  Inside a caller's
+ * stream capture a call of fewer steps than the plan's graph_chunk is captured
+ * launch by launch (a plan in the loop kernel: of any number of steps, ifdtd_plan_loop) and
+ * may be replayed while the plan, the probe and the arrays live. */
 int32_t ifdtd_step_sampled(ifdtd_plan* plan, const ifdtd_state* state, const double* currents,
                            int32_t n_steps, const ifdtd_probe* probe, double* out_rows, void* stream);
 /* Step n_steps times, sampling n_probes (1 or 2) probes after every `every`

@@ -11,7 +11,7 @@
 // (finish_grads), and one launch updates all parameters (adam_all).  At 512 traces
 // a training iteration takes 265 us instead of 1,230 (86 launches: products of
 // 22-31 us from plain loads, 24 us a column sum, host calls for each), and 4,096
-// predictions take 0.26 ms instead of 2.40, several batches sharing each launch.
+// predictions take 0.27 ms instead of 2.40, several batches sharing each launch.
 // A layer's launch still costs about 10 us of latency (launch, tensor maps, TMA,
 // epilogue), which is what bounds a pass.
 //
